@@ -7,13 +7,14 @@
 //     HBM stream instead of 8 B);
 //   * SpMV uses a sub-warp per row (width chosen from the mean row length) with shuffle
 //     reductions;
-//   * one PCG iteration is three kernels (direction update, SpMV fused with the p.q dot,
-//     vector update fused with preconditioner apply and the r.z / r.r dots); every dot is
-//     accumulated in FP64 per block and finished by the last block to arrive, in a fixed
-//     order, which also evaluates alpha / beta, breakdown and convergence on the device;
-//   * the iterations run as a CUDA graph whose 'while' node repeats a chunk of them until the
-//     device state says done; the host reads the state once, after the solve.
+//   * a CG / PCG solve is one cooperative kernel where that is the faster form (pcg_row_kernel,
+//     pcg_loop_kernel): SpMV with the p.q dot, vector update with preconditioner apply and the
+//     r.z / r.r dots, direction, with grid barriers between.  Elsewhere the same three steps are
+//     kernels, repeated by a CUDA graph 'while' node; every dot is accumulated in FP64 per block
+//     and finished by the last block to arrive, in a fixed order.  Either way the device decides
+//     when the solve is done and the host reads the state once, after it.
 #include "pm_common.cuh"
+#include "pm_grid.cuh"
 
 #include <cmath>
 #include <limits>
@@ -94,11 +95,10 @@ __global__ void validate_csr_kernel(int64_t rows, int64_t cols, int64_t nnz, con
     }
 }
 
-// y = A x with a TPR-wide sub-warp per row
-template <typename T, int TPR>
+// row of A x with a TPR-wide sub-warp per row; x_at(c) is entry c of x
+template <typename T, int TPR, typename Gather>
 __device__ __forceinline__ T csr_row_dot(const int* __restrict__ rp, const int* __restrict__ ci,
-                                         const T* __restrict__ v, const T* __restrict__ x, int64_t row, bool valid,
-                                         int lane)
+                                         const T* __restrict__ v, Gather&& x_at, int64_t row, bool valid, int lane)
 {
     T sum = T(0);
     if (valid)
@@ -123,7 +123,7 @@ __device__ __forceinline__ T csr_row_dot(const int* __restrict__ rp, const int* 
 #pragma unroll
                 for (int k = 0; k < G; ++k)
                     if (base + k < e)
-                        xv[k] = __ldg(x + col[k]);
+                        xv[k] = x_at(col[k]);
 #pragma unroll
                 for (int k = 0; k < G; ++k)
                     if (base + k < e)
@@ -133,13 +133,171 @@ __device__ __forceinline__ T csr_row_dot(const int* __restrict__ rp, const int* 
         else
         {
             for (int p = b + lane; p < e; p += TPR)
-                sum += v[p] * __ldg(x + ci[p]);
+                sum += v[p] * x_at(ci[p]);
         }
     }
 #pragma unroll
     for (int o = TPR / 2; o > 0; o >>= 1)
         sum += __shfl_xor_sync(0xffffffffu, sum, o, TPR);
     return sum;
+}
+
+// ------------------------------------------------------------------ staged row tiles
+// One lane per row with the matrix staged in shared memory.  A warp takes tiles of 32 consecutive
+// rows; the tile's nonzeros are one contiguous range of columns and values, brought in by 16-byte
+// asynchronous copies (coalesced, two tiles in flight per warp, marked evict-first in L2 so that
+// the vectors stay), and lane i then sums row i in storage order from shared memory.  Reading the
+// same rows directly costs a lane-strided access per nonzero: 180 load wavefronts per 32 rows of
+// seven FP64 nonzeros against about 100 here, and at 180 the load pipe (45 us for the 128^3
+// Laplacian) is slower than HBM.
+constexpr int kTileCap = 256; // most staged nonzeros per tile; longer tiles are taken in pieces
+template <typename T, int CAP>
+struct alignas(16) RowTile
+{
+    static_assert(CAP % 4 == 0, "whole 16-byte pieces");
+    T val[CAP];
+    int col[CAP];
+};
+
+__device__ __forceinline__ uint64_t evict_first_policy()
+{
+    uint64_t policy;
+    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;\n" : "=l"(policy));
+    return policy;
+}
+
+// 16 bytes global -> shared, of which the first `bytes` are read and the rest zero-filled
+__device__ __forceinline__ void cp_async16_stream(void* dst, const void* src, int bytes, uint64_t policy)
+{
+    asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2, %3;\n" ::"r"(smem_addr(dst)), "l"(src),
+                 "r"(bytes), "l"(policy)
+                 : "memory");
+}
+
+// nonzeros [first, first + count) into the tile (first a multiple of four, count <= its capacity);
+// nothing at or past `nnz` is read
+template <typename T, int CAP>
+__device__ __forceinline__ void tile_load(RowTile<T, CAP>& tile, const int* __restrict__ ci, const T* __restrict__ v,
+                                          int first, int count, int nnz, uint64_t policy, int lane)
+{
+    constexpr int kPer = 16 / static_cast<int>(sizeof(T));
+#pragma unroll
+    for (int u = 0; u < (CAP + 127) / 128; ++u)
+    {
+        const int k = (u * 32 + lane) * 4;
+        if (k < count)
+            cp_async16_stream(tile.col + k, ci + first + k, min(16, (nnz - first - k) * 4), policy);
+    }
+#pragma unroll
+    for (int u = 0; u < (CAP + 32 * kPer - 1) / (32 * kPer); ++u)
+    {
+        const int k = (u * 32 + lane) * kPer;
+        if (k < count)
+            cp_async16_stream(tile.val + k, v + first + k,
+                              min(16, (nnz - first - k) * static_cast<int>(sizeof(T))), policy);
+    }
+}
+
+// sum + the products of the staged positions [lo, hi), in order; gathers in groups of eight
+template <typename T, int CAP, typename Gather>
+__device__ __forceinline__ T tile_sum(const RowTile<T, CAP>& tile, int lo, int hi, T sum, Gather&& x_at)
+{
+    constexpr int G = 8;
+    for (int base = lo; base < hi; base += G)
+    {
+        T xv[G];
+#pragma unroll
+        for (int k = 0; k < G; ++k)
+            if (base + k < hi)
+                xv[k] = x_at(tile.col[base + k]);
+#pragma unroll
+        for (int k = 0; k < G; ++k)
+            if (base + k < hi)
+                sum += tile.val[base + k] * xv[k];
+    }
+    return sum;
+}
+
+// the row [b, e) of a tile whose nonzeros are [first, end), its first piece staged; tiles longer
+// than the capacity load their other pieces here
+template <typename T, int CAP, typename Gather>
+__device__ __forceinline__ T tile_row(RowTile<T, CAP>& tile, const int* __restrict__ ci, const T* __restrict__ v,
+                                      int b, int e, int first, int end, int nnz, uint64_t policy, int lane,
+                                      Gather&& x_at)
+{
+    T sum = tile_sum(tile, b - first, min(e - first, CAP), T(0), x_at);
+    for (int at = first + CAP; at < end; at += CAP)
+    {
+        __syncwarp();
+        tile_load(tile, ci, v, at, min(end - at, CAP), nnz, policy, lane);
+        cp_async_commit();
+        cp_async_wait<0>();
+        __syncwarp();
+        sum = tile_sum(tile, max(b - at, 0), min(e - at, CAP), sum, x_at);
+    }
+    return sum;
+}
+
+// Every tile warp0, warp0 + warps, ...: done(row, sum) for each of its rows, by the row's lane.
+// Values and columns 16-byte aligned; `stage`: the warp's two tiles.
+template <typename T, int CAP, typename Gather, typename Done>
+__device__ __forceinline__ void csr_tiles(RowTile<T, CAP>* stage, int64_t rows, int nnz, const int* __restrict__ rp,
+                                          const int* __restrict__ ci, const T* __restrict__ v, int64_t warp0,
+                                          int64_t warps, Gather&& x_at, Done&& done)
+{
+    const int lane = threadIdx.x & 31;
+    const uint64_t policy = evict_first_policy();
+    const int64_t tiles = (rows + 31) / 32;
+    auto bounds = [&](int64_t tile, int& b, int& e) {
+        const int64_t row = tile * 32 + lane;
+        b = e = nnz;
+        if (row < rows)
+        {
+            b = rp[row];
+            e = rp[row + 1];
+        }
+    };
+    auto issue = [&](RowTile<T, CAP>& tile, int b, int e) {
+        const int first = __shfl_sync(0xffffffffu, b, 0) & ~3;
+        const int count = __shfl_sync(0xffffffffu, e, 31) - first;
+        tile_load(tile, ci, v, first, min(count, CAP), nnz, policy, lane);
+        cp_async_commit();
+    };
+    int b, e, nb, ne, buffer = 0;
+    bounds(warp0, b, e);
+    bounds(warp0 + warps, nb, ne);
+    issue(stage[0], b, e);
+    for (int64_t t = warp0; t < tiles; t += warps)
+    {
+        issue(stage[buffer ^ 1], nb, ne);
+        int fb, fe;
+        bounds(t + 2 * warps, fb, fe);
+        cp_async_wait<1>();
+        __syncwarp();
+        const int first = __shfl_sync(0xffffffffu, b, 0) & ~3;
+        const int end = __shfl_sync(0xffffffffu, e, 31);
+        const T sum = tile_row(stage[buffer], ci, v, b, e, first, end, nnz, policy, lane, x_at);
+        if (t * 32 + lane < rows)
+            done(t * 32 + lane, sum);
+        __syncwarp();
+        b = nb;
+        e = ne;
+        nb = fb;
+        ne = fe;
+        buffer ^= 1;
+    }
+    cp_async_wait<0>();
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256, 4) csr_tile_kernel(int64_t rows, int nnz, const int* __restrict__ rp,
+                                                          const int* __restrict__ ci, const T* __restrict__ v,
+                                                          const T* __restrict__ x, T* __restrict__ y)
+{
+    extern __shared__ __align__(16) unsigned char tile_smem[];
+    csr_tiles(reinterpret_cast<RowTile<T, kTileCap>*>(tile_smem) + 2 * (threadIdx.x >> 5), rows, nnz, rp, ci, v, (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5,
+                 int64_t(gridDim.x) * (blockDim.x >> 5), [&](int c) { return __ldg(x + c); },
+                 [&](int64_t row, T sum) { y[row] = sum; });
 }
 
 // Row-group stream (chosen by pm_csr_set_kernel or the autotuner): a warp owns 32 consecutive rows.  Their nonzeros form one
@@ -149,10 +307,10 @@ __device__ __forceinline__ T csr_row_dot(const int* __restrict__ rp, const int* 
 constexpr int kStreamCap = 256; // staged products per warp
 constexpr int kStreamUnroll = kStreamCap / 32;
 
-template <typename T>
+template <typename T, typename Gather>
 __device__ __forceinline__ T csr_stream_rows(int64_t r0, int64_t rows, const int* __restrict__ rp,
-                                             const int* __restrict__ ci, const T* __restrict__ v,
-                                             const T* __restrict__ x, T* __restrict__ stage)
+                                             const int* __restrict__ ci, const T* __restrict__ v, Gather&& x_at,
+                                             T* __restrict__ stage)
 {
     const int lane = threadIdx.x & 31;
     const int64_t row = r0 + lane;
@@ -183,7 +341,7 @@ __device__ __forceinline__ T csr_stream_rows(int64_t r0, int64_t rows, const int
         {
             const int k = u * 32 + lane;
             if (k < n)
-                stage[k] = val[u] * __ldg(x + col[u]);
+                stage[k] = val[u] * x_at(col[u]);
         }
         __syncwarp();
         const int lo = my_begin > base ? my_begin : base;
@@ -205,7 +363,7 @@ __global__ void __launch_bounds__(256) csr_stream_kernel(int64_t rows, const int
     const int64_t warps = int64_t(gridDim.x) * 8;
     for (int64_t wrow = (int64_t(blockIdx.x) * 8 + warp) * 32; wrow < rows; wrow += warps * 32)
     {
-        const T sum = csr_stream_rows<T>(wrow, rows, rp, ci, v, x, stage[warp]);
+        const T sum = csr_stream_rows<T>(wrow, rows, rp, ci, v, [&](int c) { return __ldg(x + c); }, stage[warp]);
         if (wrow + (threadIdx.x & 31) < rows)
             y[wrow + (threadIdx.x & 31)] = sum;
     }
@@ -225,7 +383,8 @@ __global__ void __launch_bounds__(256) csr_spmv_kernel(int64_t rows, const int* 
     {
         const int64_t row = first + k * stride;
         const bool valid = row < rows;
-        const T sum = csr_row_dot<T, TPR>(rp, ci, v, x, row, valid, lane);
+        const T sum =
+            csr_row_dot<T, TPR>(rp, ci, v, [&](int c) { return __ldg(x + c); }, row, valid, lane);
         if (valid && lane == 0)
             y[row] = sum;
     }
@@ -245,6 +404,14 @@ int pick_tpr(int64_t rows, int64_t nnz)
     return tpr;
 }
 
+
+// one lane per row from staged tiles: the values (the caller's array) on a 16-byte boundary
+template <typename T>
+bool use_tiles(const pm_csr* A)
+{
+    return !use_stream(A) && lanes_per_row(A) == 1 && reinterpret_cast<uintptr_t>(A->values) % 16 == 0;
+}
+
 template <typename T>
 void launch_spmv(const pm_csr* A, const T* x, T* y, cudaStream_t stream)
 {
@@ -256,6 +423,15 @@ void launch_spmv(const pm_csr* A, const T* x, T* y, cudaStream_t stream)
     {
         csr_stream_kernel<T><<<grid_for(A->rows, 256, 1 << 20), 256, 0, stream>>>(A->rows, A->row_ptr, A->col_idx,
                                                                                     v, x, y);
+        PM_LAUNCH_CHECK();
+        return;
+    }
+    if (use_tiles<T>(A))
+    {
+        const size_t smem = size_t(block / 32) * 2 * sizeof(RowTile<T, kTileCap>);
+        allow_smem(reinterpret_cast<const void*>(csr_tile_kernel<T>), smem);
+        csr_tile_kernel<T><<<grid_for(A->rows, block, 4 * sm_count()), block, smem, stream>>>(
+            A->rows, static_cast<int>(A->nnz), A->row_ptr, A->col_idx, v, x, y);
         PM_LAUNCH_CHECK();
         return;
     }
@@ -287,11 +463,584 @@ struct PcgState
     int converged;
     int breakdown;     // 1: not SPD / non-finite step
     int nonfinite_init;
+    int timed_out;     // a grid barrier gave up
     long long jacobi_bad_row;
     unsigned int ticket[3];
     int chunks; // bodies run by the iteration graph
 };
 
+// ------------------------------------------------------------------ PCG in one launch
+// The whole solve is one cooperative kernel: the SpMV, the vector updates and the dots of every
+// iteration, with grid barriers in the place of kernel boundaries.  A graph of three kernels per
+// iteration costs 10-14 us an iteration however small the system is.  Every dot is accumulated in
+// FP64 per CTA; after the barrier each CTA sums the partials in the same fixed order, so all CTAs
+// take the same alpha, beta and decisions and no result depends on scheduling.
+//   pcg_row_kernel   up to 2,048 rows per SM, one lane per row: all vectors in registers, the
+//                    matrix in shared memory (24^3 grid FP32: 5.6 us an iteration against 12.7;
+//                    67^3 FP64: 13.2 against 23.4)
+//   pcg_loop_kernel  KEEP: larger, while the residual fits in shared memory beside the staged tiles
+//                    (128^3 FP64: 67 us an iteration against 79: no z, r out of L2, x and p in one
+//                    pass; DRAM traffic 212 MB an iteration against 308); otherwise systems of few
+//                    lanes in any SpMV shape (360 rows of 360: 9.5 us against 14.5)
+// Everything else runs the graph: with one CTA of at most 1,024 threads per SM the vector phases
+// of larger systems, and the block preconditioner's, have too few loads in flight (150^3 FP64: 145
+// us an iteration against 132; 24,000 rows of 474 in FP64: 55 against 49).
+constexpr int kLoopThreads = kGridMaxThreads;      // most threads of a CTA (one CTA per SM)
+constexpr int kRowThreads = 512;                   // most threads of a CTA with one row per thread
+constexpr int kKeepCap = 232;                      // staged nonzeros per tile beside the kept residual (7 per row)
+constexpr int kTileThreads = 640;                  // of a CTA that stages tiles of the matrix
+
+template <typename T>
+struct PcgLoop
+{
+    int64_t n;
+    int nnz;
+    const int* rp;
+    const int* ci;
+    const T* v;
+    const T* b;
+    T* x;
+    T* r[2];
+    T* z;
+    T* p[2];
+    T* q;
+    T* inv;
+    int mode; // 0: CG, 1: Jacobi, 2: the caller's block inverses
+    const T* blocks;
+    int64_t bs;
+    double relative, absolute;
+    Packet* mail;             // [2][CTA][CTA][2]
+    unsigned long long epoch; // barriers of earlier solves end below it
+    PcgState* st;
+};
+
+// preconditioned component i of the residual vector `r` (scalar Jacobi, caller blocks, none)
+template <typename T, typename R>
+__device__ __forceinline__ double apply_precond(int mode, int64_t i, R&& residual_at, const T* inv_diag,
+                                                const T* blocks, int64_t bs)
+{
+    if (mode == 1)
+        return static_cast<double>(inv_diag[i]) * residual_at(i);
+    if (mode == 2)
+    {
+        const int64_t blk = i / bs, local = i - blk * bs;
+        const T* row = blocks + blk * bs * bs + local * bs;
+        double z = 0.0;
+        for (int64_t c = 0; c < bs; ++c)
+            z += static_cast<double>(row[c]) * residual_at(blk * bs + c);
+        return z;
+    }
+    return residual_at(i);
+}
+
+// Jacobi inverse of row r: iterative_solver_kernels.cuh:104-131 semantics (sum of diagonal
+// duplicates, 16*eps*rowscale guard); invalid rows are reported (lowest row) instead of NaN markers.
+template <typename T>
+__device__ __forceinline__ void jacobi_row(int64_t r, const int* __restrict__ rp, const int* __restrict__ ci,
+                                           const T* __restrict__ v, T* inv, PcgState* st)
+{
+    double diag = 0.0, scale = 0.0;
+    bool found = false;
+    constexpr int G = 8; // loads in flight
+    const int e = rp[r + 1];
+    for (int p = rp[r]; p < e; p += G)
+    {
+        int col[G];
+        T value[G];
+#pragma unroll
+        for (int k = 0; k < G; ++k)
+            if (p + k < e)
+            {
+                col[k] = ci[p + k];
+                value[k] = v[p + k];
+            }
+#pragma unroll
+        for (int k = 0; k < G; ++k)
+            if (p + k < e)
+            {
+                scale = fmax(scale, fabs(static_cast<double>(value[k])));
+                if (col[k] == r)
+                {
+                    diag += static_cast<double>(value[k]);
+                    found = true;
+                }
+            }
+    }
+    const double threshold = Eps<T>::value * scale * 16.0;
+    const double reciprocal = 1.0 / diag;
+    if (!found || !isfinite(diag) || diag <= threshold || !isfinite(reciprocal))
+    {
+        atomicMin(&st->jacobi_bad_row, static_cast<long long>(r));
+        inv[r] = T(0);
+    }
+    else
+    {
+        inv[r] = static_cast<T>(reciprocal);
+    }
+}
+
+// alpha = rho / p.q (alphaKernel semantics, iterative_solver_kernels.cuh:169-202); the step must
+// also be representable in the vector type (the reference forms alpha in Scalar precision and
+// treats its overflow as breakdown); false on breakdown
+template <typename T>
+__device__ __forceinline__ bool pcg_alpha(double rho, double den, double& alpha)
+{
+    alpha = 0.0;
+    if (rho == 0.0 && den == 0.0)
+        return true;
+    if (!(isfinite(rho) && isfinite(den) && rho > 0.0 && den > 0.0))
+        return false;
+    alpha = rho / den;
+    return isfinite(alpha) && isfinite(static_cast<double>(static_cast<T>(alpha)));
+}
+
+// end of an iteration (total = {r.z, r.r}): true when the solve is over, otherwise beta and rho
+// are the next direction's (betaKernel semantics, iterative_solver_kernels.cuh:204-238)
+template <typename T>
+__device__ __forceinline__ bool pcg_finish(const double (&total)[2], double tolerance, int iterations,
+                                           int max_iterations, double& rho, double& beta, int& converged,
+                                           int& breakdown)
+{
+    const double next = total[0], residual = total[1];
+    if (!isfinite(residual) || residual < 0.0)
+    {
+        breakdown = 1;
+        return true;
+    }
+    if (sqrt(residual) <= tolerance)
+    {
+        converged = 1;
+        return true;
+    }
+    if (iterations >= max_iterations)
+        return true;
+    beta = 0.0;
+    if (!(rho == 0.0 && next == 0.0))
+    {
+        if (!(isfinite(rho) && isfinite(next) && rho > 0.0 && next > 0.0))
+        {
+            breakdown = 1;
+            return true;
+        }
+        beta = next / rho;
+        if (!isfinite(beta) || !isfinite(static_cast<double>(static_cast<T>(beta))))
+        {
+            breakdown = 1;
+            return true;
+        }
+    }
+    rho = next;
+    return false;
+}
+
+// every row of A x_at over the grid: done(row, sum) once per row
+// SHAPE: 0 row-group stream, 1 staged tiles (values 16-byte aligned), -1 a thread per row read
+// directly, otherwise lanes per row
+template <typename T, int SHAPE, int CAP, typename Gather, typename Done>
+__device__ __forceinline__ void for_rows(const PcgLoop<T>& a, unsigned char* smem, Gather&& x_at, Done&& done)
+{
+    const int64_t thread = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    const int64_t threads = int64_t(gridDim.x) * blockDim.x;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if constexpr (SHAPE == 1)
+    {
+        csr_tiles(reinterpret_cast<RowTile<T, CAP>*>(smem) + 2 * warp, a.n, a.nnz, a.rp, a.ci, a.v, thread >> 5,
+                  threads >> 5, x_at, done);
+    }
+    else if constexpr (SHAPE == 0)
+    {
+        T* stage = reinterpret_cast<T*>(smem) + warp * kStreamCap;
+        for (int64_t wrow = (thread >> 5) * 32; wrow < a.n; wrow += threads)
+        {
+            const T sum = csr_stream_rows<T>(wrow, a.n, a.rp, a.ci, a.v, x_at, stage);
+            if (wrow + lane < a.n)
+                done(wrow + lane, sum);
+        }
+    }
+    else
+    {
+        constexpr int TPR = SHAPE < 0 ? 1 : SHAPE;
+        const int64_t first = thread / TPR, stride = threads / TPR;
+        const int64_t span = (a.n + stride - 1) / stride; // uniform trip count keeps shuffles convergent
+        for (int64_t k = 0; k < span; ++k)
+        {
+            const int64_t row = first + k * stride;
+            const T sum = csr_row_dot<T, TPR>(a.rp, a.ci, a.v, x_at, row, row < a.n, lane % TPR);
+            if (row < a.n && lane % TPR == 0)
+                done(row, sum);
+        }
+    }
+}
+
+// Most threads of a CTA.  With one lane per row 640: 102 registers a thread (64 spill in FP64, 20%
+// slower) and 74-109 KB of tiles, which leave room for the kept residual.
+template <typename T>
+__host__ __device__ constexpr int loop_threads(int shape)
+{
+    return shape <= 1 ? kTileThreads : kLoopThreads;
+}
+
+// KEEP (one lane per row, modes 0 and 1): every CTA keeps its residual entries in shared memory and
+// the direction p = z + beta p, with the step of x along the old p, is a phase of its own.
+// Otherwise (FUSE) both happen inside the SpMV, every gathered entry of p formed from z and the old
+// p, which saves a grid barrier per iteration.  The arithmetic of every element is the same.
+template <typename T, int SHAPE, bool KEEP>
+__global__ void __launch_bounds__(loop_threads<T>(SHAPE), 1) pcg_loop_kernel(const PcgLoop<T> a)
+{
+    extern __shared__ __align__(16) unsigned char loop_smem[];
+    __shared__ GridShared shared;
+    PcgState* const st = a.st;
+    constexpr bool FUSE = !KEEP;
+    GridSync sync{a.mail, &st->timed_out, &shared, a.epoch};
+    if (threadIdx.x == 0)
+        shared.failed = 0; // read after the first barrier's __syncthreads
+    // a row's lane owns its entries in the vector phases too (block rows read their neighbours' q)
+    constexpr bool kOwnRows = SHAPE == 1 || SHAPE == -1 || SHAPE == 0;
+    constexpr int CAP = KEEP ? kKeepCap : kTileCap;
+    T* const kept = reinterpret_cast<T*>(loop_smem + (blockDim.x >> 5) * 2 * sizeof(RowTile<T, CAP>));
+    const int64_t thread = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    const int64_t threads = int64_t(gridDim.x) * blockDim.x;
+    const bool writer = thread == 0;
+    T* const x = a.x;
+    // ---- r = b - A x, z = M^-1 r, rho = r.z, ||r||^2 (the first direction is z)
+    if (a.mode == 1)
+        for (int64_t i = thread; i < a.n; i += threads)
+            jacobi_row<T>(i, a.rp, a.ci, a.v, a.inv, st);
+    for_rows<T, SHAPE, CAP>(a, loop_smem, [&](int c) { return x[c]; }, [&](int64_t row, T sum) { a.q[row] = sum; });
+    if (!grid_barrier(sync))
+        return;
+    double mine[2] = {0.0, 0.0}, total[2];
+    {
+        auto res = [&](int64_t k) {
+            return static_cast<double>(
+                static_cast<T>(static_cast<double>(a.b[k]) - static_cast<double>(a.q[k])));
+        };
+        for (int64_t i = thread; i < a.n; i += threads)
+        {
+            const double ri = res(i);
+            const T zi = static_cast<T>(apply_precond<T>(a.mode, i, res, a.inv, a.blocks, a.bs));
+            if (KEEP)
+                kept[(i / threads) * blockDim.x + threadIdx.x] = static_cast<T>(ri);
+            else
+                a.r[0][i] = static_cast<T>(ri);
+            a.z[i] = zi;
+            a.p[0][i] = zi;
+            mine[0] += ri * static_cast<double>(zi);
+            mine[1] += ri * ri;
+        }
+    }
+    if (!grid_sum<2>(sync, mine, total, true))
+        return;
+    double rho = total[0], residual = total[1], alpha = 0.0, beta = 0.0;
+    const double initial = sqrt(residual);
+    const double tolerance = fmax(a.absolute, a.relative * initial);
+    const int max_iterations = st->max_iterations;
+    int iterations = 0, converged = 0, breakdown = 0;
+    bool done = max_iterations <= 0;
+    if (writer)
+        st->initial_squared = residual;
+    if (!isfinite(residual) || residual < 0.0)
+    {
+        if (writer)
+            st->nonfinite_init = 1;
+        done = true;
+    }
+    else if (initial <= tolerance)
+    {
+        converged = 1;
+        done = true;
+    }
+    if (__ldcg(&st->jacobi_bad_row) != kNone)
+        done = true;
+    // ---- iterations: p0 holds the direction (FUSE: the old one once z is newer), r_in the residual
+    T *r_in = a.r[0], *r_out = a.r[1], *p0 = a.p[0], *p1 = a.p[1];
+    while (!done)
+    {
+        // direction p = z + beta p, with the step x += alpha p of the iteration before
+        if (!FUSE && iterations > 0)
+        {
+            // z is r or inv r: formed again instead of stored and read back
+            const T* own = kept + threadIdx.x;
+#pragma unroll 4
+            for (int64_t i = thread; i < a.n; i += threads, own += blockDim.x)
+            {
+                const double pi = static_cast<double>(p0[i]);
+                const double ri = static_cast<double>(*own);
+                const double zi =
+                    a.mode == 1 ? static_cast<double>(static_cast<T>(static_cast<double>(a.inv[i]) * ri)) : ri;
+                x[i] = static_cast<T>(static_cast<double>(x[i]) + alpha * pi);
+                p0[i] = static_cast<T>(zi + beta * pi);
+            }
+            if (!grid_barrier(sync))
+                return;
+        }
+        // q = A p and p.q
+        double pq[1] = {0.0}, pq_total[1];
+        if (FUSE && iterations > 0)
+        {
+            const T* const z = a.z;
+            for_rows<T, SHAPE, CAP>(
+                a, loop_smem,
+                [&](int c) { return static_cast<T>(static_cast<double>(z[c]) + beta * static_cast<double>(p0[c])); },
+                [&](int64_t row, T sum) {
+                    const double old = static_cast<double>(p0[row]);
+                    const T pn = static_cast<T>(static_cast<double>(z[row]) + beta * old);
+                    x[row] = static_cast<T>(static_cast<double>(x[row]) + alpha * old);
+                    p1[row] = pn;
+                    a.q[row] = sum;
+                    pq[0] += static_cast<double>(pn) * static_cast<double>(sum);
+                });
+            T* const t = p0;
+            p0 = p1;
+            p1 = t;
+        }
+        else
+        {
+            for_rows<T, SHAPE, CAP>(a, loop_smem, [&](int c) { return p0[c]; }, [&](int64_t row, T sum) {
+                a.q[row] = sum;
+                pq[0] += static_cast<double>(p0[row]) * static_cast<double>(sum);
+            });
+        }
+        if (!grid_sum<1>(sync, pq, pq_total, !kOwnRows || a.mode == 2))
+            return;
+        if (!pcg_alpha<T>(rho, pq_total[0], alpha))
+        {
+            breakdown = 1;
+            break; // x keeps the last completed step
+        }
+        // r -= alpha q, z = M^-1 r, r.z, r.r (r is ping-ponged: block rows read the old values)
+        mine[0] = mine[1] = 0.0;
+        if (a.mode == 2)
+        {
+            auto res = [&](int64_t k) {
+                return static_cast<double>(
+                    static_cast<T>(static_cast<double>(r_in[k]) - alpha * static_cast<double>(a.q[k])));
+            };
+            for (int64_t i = thread; i < a.n; i += threads)
+            {
+                const double ri = res(i);
+                const T zi = static_cast<T>(apply_precond<T>(a.mode, i, res, a.inv, a.blocks, a.bs));
+                r_out[i] = static_cast<T>(ri);
+                a.z[i] = zi;
+                mine[0] += ri * static_cast<double>(zi);
+                mine[1] += ri * ri;
+            }
+        }
+        else
+        {
+            T* own = kept + threadIdx.x;
+#pragma unroll 4
+            for (int64_t i = thread; i < a.n; i += threads, own += blockDim.x)
+            {
+                const T rt = static_cast<T>(static_cast<double>(KEEP ? *own : r_in[i]) -
+                                            alpha * static_cast<double>(a.q[i]));
+                const double ri = static_cast<double>(rt);
+                const T zi = a.mode == 1 ? static_cast<T>(static_cast<double>(a.inv[i]) * ri) : rt;
+                if (KEEP)
+                    *own = rt;
+                else
+                    r_out[i] = rt;
+                if (FUSE)
+                    a.z[i] = zi;
+                mine[0] += ri * static_cast<double>(zi);
+                mine[1] += ri * ri;
+            }
+        }
+        if (!grid_sum<2>(sync, mine, total, true))
+            return;
+        T* const swap = r_in;
+        r_in = r_out;
+        r_out = swap;
+        iterations += 1;
+        residual = total[1];
+        done = pcg_finish<T>(total, tolerance, iterations, max_iterations, rho, beta, converged, breakdown);
+        if (done) // the step of the last iteration
+            for (int64_t i = thread; i < a.n; i += threads)
+                x[i] = static_cast<T>(static_cast<double>(x[i]) + alpha * static_cast<double>(p0[i]));
+    }
+    if (writer)
+    {
+        st->residual_squared = residual;
+        st->iterations = iterations;
+        st->converged = converged;
+        st->breakdown = breakdown;
+    }
+}
+
+// Small systems, R rows per thread, modes 0 and 1: the matrix stays in shared memory and every
+// vector entry in its row's registers through all iterations; only z and p go through L2, for the
+// gathers.  Two barriers per iteration, as with FUSE, and the same arithmetic.
+template <typename T, int R>
+__global__ void __launch_bounds__(kRowThreads, 1) pcg_row_kernel(const PcgLoop<T> a)
+{
+    extern __shared__ __align__(16) unsigned char loop_smem[];
+    __shared__ GridShared shared;
+    PcgState* const st = a.st;
+    GridSync sync{a.mail, &st->timed_out, &shared, a.epoch};
+    if (threadIdx.x == 0)
+        shared.failed = 0; // read after the first barrier's __syncthreads
+    const int lane = threadIdx.x & 31;
+    // the warp's 32 R consecutive rows, 32 apart in a lane
+    const int64_t row0 = ((int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5) * (32 * R) + lane;
+    RowTile<T, kTileCap * R>& tile = reinterpret_cast<RowTile<T, kTileCap * R>*>(loop_smem)[threadIdx.x >> 5];
+    int b[R], e[R];
+    T x[R], inv[R], r[R], z[R], p[R], q[R];
+#pragma unroll
+    for (int j = 0; j < R; ++j)
+    {
+        const int64_t row = row0 + 32 * j;
+        b[j] = row < a.n ? a.rp[row] : a.nnz;
+        e[j] = row < a.n ? a.rp[row + 1] : a.nnz;
+    }
+    const int first = __shfl_sync(0xffffffffu, b[0], 0), end = __shfl_sync(0xffffffffu, e[R - 1], 31);
+    const bool staged = end - first <= kTileCap * R; // otherwise the rows are read directly
+    if (staged)
+    {
+        for (int k = lane; k < end - first; k += 32)
+        {
+            tile.col[k] = a.ci[first + k];
+            tile.val[k] = a.v[first + k];
+        }
+#pragma unroll
+        for (int j = 0; j < R; ++j)
+        {
+            b[j] -= first;
+            e[j] -= first;
+        }
+    }
+    __syncwarp();
+    auto row_sums = [&](auto&& x_at) {
+#pragma unroll
+        for (int j = 0; j < R; ++j)
+        {
+            q[j] = T(0);
+            if (staged)
+                q[j] = tile_sum(tile, b[j], e[j], T(0), x_at);
+            else
+                for (int k = b[j]; k < e[j]; ++k)
+                    q[j] += a.v[k] * x_at(a.ci[k]);
+        }
+    };
+    T* const z_all = a.z;
+    T *p_old = a.p[0], *p_new = a.p[1];
+    double mine[2] = {0.0, 0.0}, total[2];
+    row_sums([&](int c) { return a.x[c]; });
+#pragma unroll
+    for (int j = 0; j < R; ++j)
+    {
+        const int64_t row = row0 + 32 * j;
+        x[j] = r[j] = z[j] = p[j] = T(0);
+        inv[j] = T(1);
+        if (row < a.n)
+        {
+            if (a.mode == 1)
+            {
+                jacobi_row<T>(row, a.rp, a.ci, a.v, a.inv, st);
+                inv[j] = a.inv[row];
+            }
+            x[j] = a.x[row];
+            r[j] = static_cast<T>(static_cast<double>(a.b[row]) - static_cast<double>(q[j]));
+            const double ri = static_cast<double>(r[j]);
+            p[j] = z[j] = a.mode == 1 ? static_cast<T>(static_cast<double>(inv[j]) * ri) : r[j];
+            p_old[row] = z[j];
+            mine[0] += ri * static_cast<double>(z[j]);
+            mine[1] += ri * ri;
+        }
+    }
+    if (!grid_sum<2>(sync, mine, total, true))
+        return;
+    double rho = total[0], residual = total[1], beta = 0.0;
+    const double initial = sqrt(residual);
+    const double tolerance = fmax(a.absolute, a.relative * initial);
+    const int max_iterations = st->max_iterations;
+    int iterations = 0, converged = 0, breakdown = 0;
+    bool done = max_iterations <= 0;
+    const bool writer = blockIdx.x == 0 && threadIdx.x == 0;
+    if (writer)
+        st->initial_squared = residual;
+    if (!isfinite(residual) || residual < 0.0)
+    {
+        if (writer)
+            st->nonfinite_init = 1;
+        done = true;
+    }
+    else if (initial <= tolerance)
+    {
+        converged = 1;
+        done = true;
+    }
+    if (__ldcg(&st->jacobi_bad_row) != kNone)
+        done = true;
+    while (!done)
+    {
+        if (iterations == 0)
+        {
+            row_sums([&](int c) { return p_old[c]; });
+        }
+        else
+        {
+            row_sums([&](int c) {
+                return static_cast<T>(static_cast<double>(z_all[c]) + beta * static_cast<double>(p_old[c]));
+            });
+#pragma unroll
+            for (int j = 0; j < R; ++j)
+            {
+                p[j] = static_cast<T>(static_cast<double>(z[j]) + beta * static_cast<double>(p[j]));
+                if (row0 + 32 * j < a.n)
+                    p_new[row0 + 32 * j] = p[j];
+            }
+            T* const t = p_old;
+            p_old = p_new;
+            p_new = t;
+        }
+        double pq[1] = {0.0}, pq_total[1];
+#pragma unroll
+        for (int j = 0; j < R; ++j) // rows past the end hold zeros
+            pq[0] += static_cast<double>(p[j]) * static_cast<double>(q[j]);
+        if (!grid_sum<1>(sync, pq, pq_total, false))
+            return;
+        double alpha;
+        if (!pcg_alpha<T>(rho, pq_total[0], alpha))
+        {
+            breakdown = 1;
+            break;
+        }
+        mine[0] = mine[1] = 0.0;
+#pragma unroll
+        for (int j = 0; j < R; ++j)
+        {
+            r[j] = static_cast<T>(static_cast<double>(r[j]) - alpha * static_cast<double>(q[j]));
+            const double ri = static_cast<double>(r[j]);
+            z[j] = a.mode == 1 ? static_cast<T>(static_cast<double>(inv[j]) * ri) : r[j];
+            x[j] = static_cast<T>(static_cast<double>(x[j]) + alpha * static_cast<double>(p[j]));
+            if (row0 + 32 * j < a.n)
+                z_all[row0 + 32 * j] = z[j];
+            mine[0] += ri * static_cast<double>(z[j]);
+            mine[1] += ri * ri;
+        }
+        if (!grid_sum<2>(sync, mine, total, true))
+            return;
+        iterations += 1;
+        residual = total[1];
+        done = pcg_finish<T>(total, tolerance, iterations, max_iterations, rho, beta, converged, breakdown);
+    }
+    if (iterations > 0)
+    {
+#pragma unroll
+        for (int j = 0; j < R; ++j)
+            if (row0 + 32 * j < a.n)
+                a.x[row0 + 32 * j] = x[j];
+    }
+    if (writer)
+    {
+        st->residual_squared = residual;
+        st->iterations = iterations;
+        st->converged = converged;
+        st->breakdown = breakdown;
+    }
+}
+
+// ------------------------------------------------------------------ PCG as a graph of kernels
 // Last block to arrive sums the per-block partials (fixed order) and runs `finish`.
 template <int K, typename Finish>
 __device__ __forceinline__ void reduce_partials(double (&mine)[K], double* partials, unsigned int* ticket,
@@ -329,57 +1078,12 @@ __device__ __forceinline__ void reduce_partials(double (&mine)[K], double* parti
     }
 }
 
-// preconditioned component i of the residual vector `r` (scalar Jacobi, caller blocks, none)
-template <typename T, typename R>
-__device__ __forceinline__ double apply_precond(int mode, int64_t i, R&& residual_at, const T* inv_diag,
-                                                const T* blocks, int64_t bs)
-{
-    if (mode == 1)
-        return static_cast<double>(inv_diag[i]) * residual_at(i);
-    if (mode == 2)
-    {
-        const int64_t blk = i / bs, local = i - blk * bs;
-        const T* row = blocks + blk * bs * bs + local * bs;
-        double z = 0.0;
-        for (int64_t c = 0; c < bs; ++c)
-            z += static_cast<double>(row[c]) * residual_at(blk * bs + c);
-        return z;
-    }
-    return residual_at(i);
-}
-
-// Jacobi inverse: iterative_solver_kernels.cuh:104-131 semantics (sum of diagonal duplicates,
-// 16*eps*rowscale guard); invalid rows are reported (lowest row) instead of NaN markers.
 template <typename T>
 __global__ void jacobi_kernel(int64_t rows, const int* __restrict__ rp, const int* __restrict__ ci,
                               const T* __restrict__ v, T* __restrict__ inv, PcgState* st)
 {
     for (int64_t r = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; r < rows; r += int64_t(gridDim.x) * blockDim.x)
-    {
-        double diag = 0.0, scale = 0.0;
-        bool found = false;
-        for (int p = rp[r]; p < rp[r + 1]; ++p)
-        {
-            const double value = static_cast<double>(v[p]);
-            scale = fmax(scale, fabs(value));
-            if (ci[p] == r)
-            {
-                diag += value;
-                found = true;
-            }
-        }
-        const double threshold = Eps<T>::value * scale * 16.0;
-        const double reciprocal = 1.0 / diag;
-        if (!found || !isfinite(diag) || diag <= threshold || !isfinite(reciprocal))
-        {
-            atomicMin(&st->jacobi_bad_row, static_cast<long long>(r));
-            inv[r] = T(0);
-        }
-        else
-        {
-            inv[r] = static_cast<T>(reciprocal);
-        }
-    }
+        jacobi_row<T>(r, rp, ci, v, inv, st);
 }
 
 // r = b - Ax (Ax in q), z = M^-1 r, p = z; rho = r.z, initial ||r||^2
@@ -426,35 +1130,21 @@ __global__ void __launch_bounds__(kReduceBlock) pcg_init_kernel(int64_t n, const
     });
 }
 
-// alpha = rho / p.q on the last block (alphaKernel semantics, iterative_solver_kernels.cuh:169-202)
+// alpha = rho / p.q on the last block
 template <typename T>
-__device__ __forceinline__ void pcg_alpha(PcgState* st, double den, T)
+__device__ __forceinline__ void pcg_step(PcgState* st, double den, T)
 {
-    const double rho = st->rho;
-    double alpha = 0.0;
-    if (rho == 0.0 && den == 0.0)
-        alpha = 0.0;
-    else if (isfinite(rho) && isfinite(den) && rho > 0.0 && den > 0.0)
-    {
-        alpha = rho / den;
-        // the step must also be representable in the vector type (the reference forms
-        // alpha in Scalar precision and treats its overflow as breakdown)
-        if (!isfinite(alpha) || !isfinite(static_cast<double>(static_cast<T>(alpha))))
-        {
-            st->breakdown = 1;
-            alpha = 0.0;
-        }
-    }
-    else
+    double alpha;
+    if (!pcg_alpha<T>(st->rho, den, alpha))
     {
         st->breakdown = 1;
+        st->done = 1;
+        alpha = 0.0;
     }
     st->alpha = alpha;
-    if (st->breakdown)
-        st->done = 1;
 }
 
-// q = A p, alpha = rho / p.q  (alphaKernel semantics, iterative_solver_kernels.cuh:169-202)
+// q = A p, alpha = rho / p.q
 template <typename T, int TPR>
 __global__ void __launch_bounds__(kReduceBlock) pcg_spmv_kernel(int64_t rows, const int* __restrict__ rp,
                                                                 const int* __restrict__ ci, const T* __restrict__ v,
@@ -472,14 +1162,14 @@ __global__ void __launch_bounds__(kReduceBlock) pcg_spmv_kernel(int64_t rows, co
     {
         const int64_t row = first + k * stride;
         const bool valid = row < rows;
-        const T sum = csr_row_dot<T, TPR>(rp, ci, v, p, row, valid, lane);
+        const T sum = csr_row_dot<T, TPR>(rp, ci, v, [&](int c) { return __ldg(p + c); }, row, valid, lane);
         if (valid && lane == 0)
         {
             q[row] = sum;
             mine[0] += static_cast<double>(p[row]) * static_cast<double>(sum);
         }
     }
-    reduce_partials<1>(mine, partials, &st->ticket[1], [&](double (&tot)[1]) { pcg_alpha(st, tot[0], T(0)); });
+    reduce_partials<1>(mine, partials, &st->ticket[1], [&](double (&tot)[1]) { pcg_step(st, tot[0], T(0)); });
 }
 
 // q = A p with the short-row stream layout, alpha = rho / p.q
@@ -498,7 +1188,7 @@ __global__ void __launch_bounds__(kReduceBlock) pcg_stream_spmv_kernel(int64_t r
     const int64_t warps = int64_t(gridDim.x) * (kReduceBlock / 32);
     for (int64_t wrow = (int64_t(blockIdx.x) * (kReduceBlock / 32) + warp) * 32; wrow < rows; wrow += warps * 32)
     {
-        const T sum = csr_stream_rows<T>(wrow, rows, rp, ci, v, p, stage[warp]);
+        const T sum = csr_stream_rows<T>(wrow, rows, rp, ci, v, [&](int c) { return __ldg(p + c); }, stage[warp]);
         const int64_t row = wrow + lane;
         if (row < rows)
         {
@@ -506,7 +1196,29 @@ __global__ void __launch_bounds__(kReduceBlock) pcg_stream_spmv_kernel(int64_t r
             mine[0] += static_cast<double>(p[row]) * static_cast<double>(sum);
         }
     }
-    reduce_partials<1>(mine, partials, &st->ticket[1], [&](double (&tot)[1]) { pcg_alpha(st, tot[0], T(0)); });
+    reduce_partials<1>(mine, partials, &st->ticket[1], [&](double (&tot)[1]) { pcg_step(st, tot[0], T(0)); });
+}
+
+// q = A p from staged tiles, alpha = rho / p.q
+template <typename T>
+__global__ void __launch_bounds__(kReduceBlock, 4) pcg_tile_spmv_kernel(int64_t rows, int nnz,
+                                                                        const int* __restrict__ rp,
+                                                                        const int* __restrict__ ci,
+                                                                        const T* __restrict__ v,
+                                                                        const T* __restrict__ p, T* __restrict__ q,
+                                                                        double* partials, PcgState* st)
+{
+    if (st->done)
+        return;
+    extern __shared__ __align__(16) unsigned char tile_smem[];
+    double mine[1] = {0.0};
+    csr_tiles(reinterpret_cast<RowTile<T, kTileCap>*>(tile_smem) + 2 * (threadIdx.x >> 5), rows, nnz, rp, ci, v,
+              (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5, int64_t(gridDim.x) * (blockDim.x >> 5),
+              [&](int c) { return __ldg(p + c); }, [&](int64_t row, T sum) {
+                  q[row] = sum;
+                  mine[0] += static_cast<double>(p[row]) * static_cast<double>(sum);
+              });
+    reduce_partials<1>(mine, partials, &st->ticket[1], [&](double (&tot)[1]) { pcg_step(st, tot[0], T(0)); });
 }
 
 // x += alpha p, r -= alpha q, z = M^-1 r; convergence on ||r||, beta = r.z / rho.
@@ -540,45 +1252,14 @@ __global__ void __launch_bounds__(kReduceBlock) pcg_update_kernel(int64_t n, T* 
     reduce_partials<2>(mine, partials, &st->ticket[2], [&](double (&tot)[2]) {
         st->iterations += 1;
         st->residual_squared = tot[1];
-        if (!isfinite(tot[1]) || tot[1] < 0.0)
-        {
-            st->breakdown = 1;
-            st->done = 1;
-            return;
-        }
-        if (sqrt(tot[1]) <= st->tolerance)
-        {
-            st->converged = 1;
-            st->done = 1;
-            return;
-        }
-        if (st->iterations >= st->max_iterations)
-        {
-            st->done = 1;
-            return;
-        }
-        // betaKernel semantics (iterative_solver_kernels.cuh:204-238)
-        const double rho = st->rho, next = tot[0];
-        double beta = 0.0;
-        if (rho == 0.0 && next == 0.0)
-            beta = 0.0;
-        else if (isfinite(rho) && isfinite(next) && rho > 0.0 && next > 0.0)
-        {
-            beta = next / rho;
-            if (!isfinite(beta) || !isfinite(static_cast<double>(static_cast<T>(beta))))
-            {
-                st->breakdown = 1;
-                st->done = 1;
-                beta = 0.0;
-            }
-        }
-        else
-        {
-            st->breakdown = 1;
-            st->done = 1;
-        }
+        double rho = st->rho, beta = st->beta;
+        int converged = 0, breakdown = 0;
+        st->done = pcg_finish<T>(tot, st->tolerance, st->iterations, st->max_iterations, rho, beta, converged,
+                                 breakdown);
+        st->rho = rho;
         st->beta = beta;
-        st->rho = next;
+        st->converged = converged;
+        st->breakdown = breakdown;
     });
 }
 
@@ -617,7 +1298,7 @@ __global__ void pcg_reset_kernel(PcgState* st, int max_iterations)
 __global__ void fixed_finish_kernel(const PcgState* st, double* out)
 {
     const double nan = __longlong_as_double(0x7ff8000000000000LL);
-    const bool bad = st->breakdown || st->nonfinite_init || st->jacobi_bad_row != kNone;
+    const bool bad = st->breakdown || st->nonfinite_init || st->timed_out || st->jacobi_bad_row != kNone;
     out[0] = st->nonfinite_init ? nan : st->initial_squared;
     out[1] = bad ? nan : st->residual_squared;
 }
@@ -643,7 +1324,8 @@ struct pm_fixed_state
 struct pm_solver_workspace
 {
     pm::DeviceBuffer buffer;
-    int* host_done = nullptr; // pinned
+    pm::GridMail mail;
+    void* host_state = nullptr; // pinned
     cudaEvent_t event = nullptr;
     // CG / PCG iteration graphs ('while' node around a chunk of iterations), one per operand set
     struct IterationGraph
@@ -675,8 +1357,9 @@ struct pm_solver_workspace
         if (capture_stream)
             cudaStreamDestroy(capture_stream);
         buffer.release();
-        if (host_done)
-            cudaFreeHost(host_done);
+        mail.buffer.release();
+        if (host_state)
+            cudaFreeHost(host_state);
         if (event)
             cudaEventDestroy(event);
     }
@@ -948,6 +1631,26 @@ void csr_spmm(const pm_csr* A, cudaStream_t stream, int64_t in_rows, int64_t in_
     PM_LAUNCH_CHECK();
 }
 
+// the workspace's arrays for a system of n rows
+template <typename T>
+struct PcgVectors
+{
+    PcgState* st;
+    double* partials;
+    T *r[2], *z, *p[2], *q, *inv;
+    size_t bytes;
+    PcgVectors(const pm_solver_workspace* ws, int64_t n)
+    {
+        Carver c;
+        c.base = static_cast<char*>(ws->buffer.ptr);
+        st = c.take<PcgState>(1);
+        partials = c.take<double>(3 * kMaxReduceBlocks);
+        for (T** v : {&r[0], &r[1], &z, &p[0], &p[1], &q, &inv})
+            *v = c.take<T>(n);
+        bytes = c.offset;
+    }
+};
+
 template <typename T>
 void launch_pcg_spmv(const pm_csr* A, const T* p, T* q, double* partials, PcgState* st, unsigned grid,
                      cudaStream_t stream)
@@ -957,6 +1660,17 @@ void launch_pcg_spmv(const pm_csr* A, const T* p, T* q, double* partials, PcgSta
     {
         pcg_stream_spmv_kernel<T><<<grid, kReduceBlock, 0, stream>>>(A->rows, A->row_ptr, A->col_idx, v, p, q,
                                                                      partials, st);
+        PM_LAUNCH_CHECK();
+        return;
+    }
+    // FP32 only: in FP64 the tiles' 197 KB of shared memory leave the gathers of p too little L1
+    // (150^3: 4.12 ms for 30 iterations against 4.00 read directly; FP32 2.76 against 3.16)
+    if (sizeof(T) == 4 && use_tiles<T>(A))
+    {
+        const size_t smem = size_t(kReduceBlock / 32) * 2 * sizeof(RowTile<T, kTileCap>);
+        allow_smem(reinterpret_cast<const void*>(pcg_tile_spmv_kernel<T>), smem);
+        pcg_tile_spmv_kernel<T><<<std::min<unsigned>(grid, 4 * sm_count()), kReduceBlock, smem, stream>>>(
+            A->rows, static_cast<int>(A->nnz), A->row_ptr, A->col_idx, v, p, q, partials, st);
         PM_LAUNCH_CHECK();
         return;
     }
@@ -996,16 +1710,10 @@ cudaGraphExec_t cg_iteration_graph(pm_solver_workspace* ws, const pm_csr* A, T* 
     if (slot.graph)
         cudaGraphDestroy(slot.graph);
     slot = pm_solver_workspace::IterationGraph{};
-    Carver c;
-    c.base = static_cast<char*>(ws->buffer.ptr);
-    PcgState* st = c.take<PcgState>(1);
-    double* partials = c.take<double>(3 * kMaxReduceBlocks);
-    T* r0 = c.take<T>(n);
-    T* r1 = c.take<T>(n);
-    T* z = c.take<T>(n);
-    T* p = c.take<T>(n);
-    T* q = c.take<T>(n);
-    T* inv = c.take<T>(n);
+    const PcgVectors<T> u(ws, n);
+    PcgState* const st = u.st;
+    double* const partials = u.partials;
+    T *const r0 = u.r[0], *const r1 = u.r[1], *const z = u.z, *const p = u.p[0], *const q = u.q, *const inv = u.inv;
     const unsigned vgrid = grid_for(n, kReduceBlock, kMaxReduceBlocks);
     const unsigned sgrid = use_stream(A) ? grid_for(n, kReduceBlock, kMaxReduceBlocks)
                                          : grid_for(n * lanes_per_row(A), kReduceBlock, kMaxReduceBlocks);
@@ -1062,6 +1770,135 @@ cudaGraphExec_t cg_iteration_graph(pm_solver_workspace* ws, const pm_csr* A, T* 
     return exec;
 }
 
+template <typename T, typename Kernel>
+void launch_cooperative(Kernel kernel, PcgLoop<T>& a, unsigned ctas, unsigned threads, size_t smem, cudaStream_t stream)
+{
+    allow_smem(reinterpret_cast<const void*>(kernel), smem);
+    void* args[] = {&a};
+    PM_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), dim3(ctas), dim3(threads), args, smem,
+                                        stream));
+    PM_LAUNCH_CHECK();
+}
+
+// One cooperative launch of the whole solve where it is the faster form (see pcg_loop_kernel);
+// false where it is not.  One CTA per SM at most: they wait for one another, so all must be resident.
+template <typename T, int SHAPE>
+bool launch_pcg_loop_shape(PcgLoop<T>& a, size_t warp_smem, int lanes, cudaStream_t stream)
+{
+    const int most = std::min(sm_count(), kGridMaxCtas);
+    if constexpr (SHAPE == 1)
+    {
+        constexpr size_t kSmem = 226 * 1024; // of the 227 KB a CTA may have; the rest is static
+        if (a.mode != 2 && a.n <= int64_t(4) * kRowThreads * most)
+        {
+            const auto launch_rows = [&](auto kernel, int per_thread) {
+                unsigned block = 256;
+                if (a.n > int64_t(block) * per_thread * most)
+                    block = kRowThreads;
+                launch_cooperative(kernel, a, grid_for(a.n, static_cast<int>(block) * per_thread, most), block,
+                                   size_t(kTileCap) * per_thread * (sizeof(T) + sizeof(int)) * (block / 32), stream);
+                return true;
+            };
+            if (a.n <= int64_t(kRowThreads) * most)
+                return launch_rows(pcg_row_kernel<T, 1>, 1);
+            if (a.n <= int64_t(2) * kRowThreads * most)
+                return launch_rows(pcg_row_kernel<T, 2>, 2);
+            return launch_rows(pcg_row_kernel<T, 4>, 4);
+        }
+        const unsigned ctas = grid_for(a.n, kTileThreads, most);
+        const int64_t per_thread = (a.n + int64_t(ctas) * kTileThreads - 1) / (int64_t(ctas) * kTileThreads);
+        const size_t kept = size_t(per_thread) * kTileThreads * sizeof(T);
+        const size_t staged = kTileThreads / 32 * 2 * sizeof(RowTile<T, kKeepCap>);
+        if (a.mode != 2 && kept <= kSmem - staged)
+        {
+            launch_cooperative(pcg_loop_kernel<T, 1, true>, a, ctas, kTileThreads, staged + kept, stream);
+            return true;
+        }
+        warp_smem = 2 * sizeof(RowTile<T, kTileCap>);
+    }
+    // few lanes: one row per thread (or group of lanes)
+    constexpr unsigned kMost = loop_threads<T>(SHAPE);
+    const int64_t wanted = a.n * lanes;
+    if (wanted > int64_t(kMost) * most)
+        return false;
+    unsigned threads = 256;
+    while (threads < kMost && wanted > int64_t(threads) * most)
+        threads = std::min(2 * threads, kMost);
+    launch_cooperative(pcg_loop_kernel<T, SHAPE, false>, a, grid_for(wanted, static_cast<int>(threads), most), threads,
+                       warp_smem * (threads / 32), stream);
+    return true;
+}
+
+template <typename T>
+bool launch_pcg_loop(const pm_csr* A, PcgLoop<T>& a, cudaStream_t stream)
+{
+    if (use_stream(A))
+        return launch_pcg_loop_shape<T, 0>(a, kStreamCap * sizeof(T), 1, stream);
+    if (use_tiles<T>(A))
+        return launch_pcg_loop_shape<T, 1>(a, 0, 1, stream);
+    switch (lanes_per_row(A))
+    {
+    case 1: return launch_pcg_loop_shape<T, -1>(a, 0, 1, stream);
+    case 2: return launch_pcg_loop_shape<T, 2>(a, 0, 2, stream);
+    case 4: return launch_pcg_loop_shape<T, 4>(a, 0, 4, stream);
+    case 8: return launch_pcg_loop_shape<T, 8>(a, 0, 8, stream);
+    case 16: return launch_pcg_loop_shape<T, 16>(a, 0, 16, stream);
+    default: return launch_pcg_loop_shape<T, 32>(a, 0, 32, stream);
+    }
+}
+
+// Queues a solve: one cooperative launch, or the initial residual and then the iterations as kernels
+// (from the operand set's graph, or one by one when `graph` is false).  Returns the device state.
+template <typename T>
+PcgState* queue_pcg(pm_solver_workspace* ws, const pm_csr* A, const T* b, T* x, const T* blocks, int64_t bs, int mode,
+                    double relative, double absolute, int max_iterations, bool graph, cudaStream_t stream)
+{
+    const int64_t n = A->rows;
+    ws->buffer.ensure(PcgVectors<T>(ws, n).bytes + 256, stream, "IterativeSolverWorkspace");
+    const PcgVectors<T> u(ws, n);
+    ws->mail.open(stream, "IterativeSolverWorkspace");
+    const T* v = static_cast<const T*>(A->values);
+    pcg_reset_kernel<<<1, 1, 0, stream>>>(u.st, max_iterations);
+    PM_LAUNCH_CHECK();
+    PcgLoop<T> a{n, static_cast<int>(A->nnz), A->row_ptr, A->col_idx, v, b, x, {u.r[0], u.r[1]}, u.z, {u.p[0], u.p[1]},
+                 u.q, u.inv, mode, blocks, bs, relative, absolute, ws->mail.packets(), ws->mail.epoch, u.st};
+    if (launch_pcg_loop<T>(A, a, stream))
+        return u.st;
+    if (mode == 1)
+    {
+        jacobi_kernel<T><<<grid_for(n, 256, 4096), 256, 0, stream>>>(n, A->row_ptr, A->col_idx, v, u.inv, u.st);
+        PM_LAUNCH_CHECK();
+    }
+    const unsigned vgrid = grid_for(n, kReduceBlock, kMaxReduceBlocks);
+    launch_spmv<T>(A, x, u.q, stream);
+    pcg_init_kernel<T><<<vgrid, kReduceBlock, 0, stream>>>(n, b, u.q, u.r[0], u.z, u.p[0], mode, u.inv, blocks, bs,
+                                                            relative, absolute, u.partials, u.st);
+    PM_LAUNCH_CHECK();
+    if (graph && max_iterations > 0)
+    {
+        const cudaGraphExec_t exec = cg_iteration_graph<T>(ws, A, x, blocks, bs, mode);
+        PM_CUDA(cudaMemsetAsync(&u.st->chunks, 0, sizeof(int), stream));
+        PM_CUDA(cudaGraphLaunch(exec, stream));
+    }
+    else
+    {
+        const unsigned sgrid = use_stream(A) ? vgrid : grid_for(n * lanes_per_row(A), kReduceBlock, kMaxReduceBlocks);
+        for (int k = 0; k < max_iterations; ++k)
+        {
+            if (k > 0)
+            {
+                pcg_direction_kernel<T><<<vgrid, kReduceBlock, 0, stream>>>(n, u.z, u.p[0], u.st);
+                PM_LAUNCH_CHECK();
+            }
+            launch_pcg_spmv<T>(A, u.p[0], u.q, u.partials, u.st, sgrid, stream);
+            pcg_update_kernel<T><<<vgrid, kReduceBlock, 0, stream>>>(n, x, u.p[0], u.q, u.r[k & 1], u.r[(k & 1) ^ 1],
+                                                                      u.z, mode, u.inv, blocks, bs, u.partials, u.st);
+            PM_LAUNCH_CHECK();
+        }
+    }
+    return u.st;
+}
+
 // mode: 0 = CG, 1 = Jacobi PCG, 2 = caller block inverses
 template <typename T>
 void solve(pm_solver_workspace* ws, cudaStream_t stream, const pm_csr* A, const T* b, T* x, const T* blocks,
@@ -1095,57 +1932,20 @@ void solve(pm_solver_workspace* ws, cudaStream_t stream, const pm_csr* A, const 
         report->converged = 1;
         return;
     }
-    Carver plan;
-    plan.take<PcgState>(1);
-    plan.take<double>(3 * kMaxReduceBlocks);
-    for (int k = 0; k < 6; ++k)
-        plan.take<T>(n);
-    ws->buffer.ensure(plan.offset + 256, stream, "IterativeSolverWorkspace");
-    if (!ws->host_done)
-        PM_CUDA(cudaMallocHost(reinterpret_cast<void**>(&ws->host_done), 2 * sizeof(PcgState)));
+    if (!ws->host_state)
+        PM_CUDA(cudaMallocHost(&ws->host_state, sizeof(PcgState)));
     if (!ws->event)
         PM_CUDA(cudaEventCreateWithFlags(&ws->event, cudaEventDisableTiming));
-    Carver c;
-    c.base = static_cast<char*>(ws->buffer.ptr);
-    PcgState* st = c.take<PcgState>(1);
-    double* partials = c.take<double>(3 * kMaxReduceBlocks);
-    T* r0 = c.take<T>(n);
-    T* r1 = c.take<T>(n);
-    T* z = c.take<T>(n);
-    T* p = c.take<T>(n);
-    T* q = c.take<T>(n);
-    T* inv = c.take<T>(n);
-
-    const unsigned vgrid = grid_for(n, kReduceBlock, kMaxReduceBlocks);
-    const unsigned sgrid = use_stream(A) ? grid_for(n, kReduceBlock, kMaxReduceBlocks)
-                                                   : grid_for(n * lanes_per_row(A), kReduceBlock, kMaxReduceBlocks);
-    pcg_reset_kernel<<<1, 1, 0, stream>>>(st, o->max_iterations);
-    PM_LAUNCH_CHECK();
-    if (mode == 1)
-    {
-        jacobi_kernel<T><<<grid_for(n, 256, 4096), 256, 0, stream>>>(n, A->row_ptr, A->col_idx,
-                                                                       static_cast<const T*>(A->values), inv, st);
-        PM_LAUNCH_CHECK();
-    }
-    launch_spmv<T>(A, x, q, stream);
-    pcg_init_kernel<T><<<vgrid, kReduceBlock, 0, stream>>>(n, b, q, r0, z, p, mode, inv, blocks, bs,
-                                                            o->relative_tolerance, o->absolute_tolerance, partials, st);
-    PM_LAUNCH_CHECK();
-    // the iterations: one launch of the operand set's iteration graph, which stops on the device
-    PcgState* host = reinterpret_cast<PcgState*>(ws->host_done);
-    if (o->max_iterations > 0)
-    {
-        const cudaGraphExec_t exec = cg_iteration_graph<T>(ws, A, x, blocks, bs, mode);
-        PM_CUDA(cudaMemsetAsync(&st->chunks, 0, sizeof(int), stream));
-        PM_CUDA(cudaGraphLaunch(exec, stream));
-    }
-    PM_CUDA(cudaMemcpyAsync(host, st, sizeof(PcgState), cudaMemcpyDeviceToHost, stream));
+    const PcgState* st = queue_pcg<T>(ws, A, b, x, blocks, bs, mode, o->relative_tolerance, o->absolute_tolerance,
+                                      o->max_iterations, true, stream);
+    PM_CUDA(cudaMemcpyAsync(ws->host_state, st, sizeof(PcgState), cudaMemcpyDeviceToHost, stream));
     PM_CUDA(cudaEventRecord(ws->event, stream));
     PM_CUDA(cudaEventSynchronize(ws->event));
-    if (o->max_iterations > 0) // the kernels the graph ran: three per iteration and the condition
-        for (int k = 0; k < host->chunks * (3 * kCgChunk + 1); ++k)
-            count_launch();
-    const PcgState s = *host;
+    const PcgState s = *static_cast<PcgState*>(ws->host_state);
+    for (int k = 0; k < s.chunks * (3 * kCgChunk + 1); ++k) // the kernels a graph ran
+        count_launch();
+    if (s.timed_out)
+        fail(PM_CUDA_ERROR, "CUDA iterative solver: a grid barrier did not complete");
     if (s.jacobi_bad_row != kNone)
     {
         std::ostringstream m;
@@ -1202,52 +2002,8 @@ pm_fixed_state* fixed_solve(pm_solver_workspace* ws, cudaStream_t stream, const 
             PM_CUDA(cudaEventRecord(state->event, stream));
             return state;
         }
-        Carver plan;
-        plan.take<PcgState>(1);
-        plan.take<double>(3 * kMaxReduceBlocks);
-        for (int k = 0; k < 6; ++k)
-            plan.take<T>(n);
-        ws->buffer.ensure(plan.offset + 256, stream, "IterativeSolverWorkspace");
-        Carver c;
-        c.base = static_cast<char*>(ws->buffer.ptr);
-        PcgState* st = c.take<PcgState>(1);
-        double* partials = c.take<double>(3 * kMaxReduceBlocks);
-        T* r0 = c.take<T>(n);
-        T* r1 = c.take<T>(n);
-        T* z = c.take<T>(n);
-        T* p = c.take<T>(n);
-        T* q = c.take<T>(n);
-        T* inv = c.take<T>(n);
-        const unsigned vgrid = grid_for(n, kReduceBlock, kMaxReduceBlocks);
-        const unsigned sgrid = use_stream(A) ? grid_for(n, kReduceBlock, kMaxReduceBlocks)
-                                                       : grid_for(n * lanes_per_row(A), kReduceBlock, kMaxReduceBlocks);
-        pcg_reset_kernel<<<1, 1, 0, stream>>>(st, iterations);
-        PM_LAUNCH_CHECK();
-        if (mode == 1)
-        {
-            jacobi_kernel<T><<<grid_for(n, 256, 4096), 256, 0, stream>>>(n, A->row_ptr, A->col_idx,
-                                                                           static_cast<const T*>(A->values), inv, st);
-            PM_LAUNCH_CHECK();
-        }
-        launch_spmv<T>(A, x, q, stream);
-        pcg_init_kernel<T><<<vgrid, kReduceBlock, 0, stream>>>(n, b, q, r0, z, p, mode, inv, static_cast<const T*>(nullptr),
-                                                                0, 0.0, 0.0, partials, st);
-        PM_LAUNCH_CHECK();
-        T* r_in = r0;
-        T* r_out = r1;
-        for (int k = 0; k < iterations; ++k)
-        {
-            if (k > 0)
-            {
-                pcg_direction_kernel<T><<<vgrid, kReduceBlock, 0, stream>>>(n, z, p, st);
-                PM_LAUNCH_CHECK();
-            }
-            launch_pcg_spmv<T>(A, p, q, partials, st, sgrid, stream);
-            pcg_update_kernel<T><<<vgrid, kReduceBlock, 0, stream>>>(n, x, p, q, r_in, r_out, z, mode, inv,
-                                                                      static_cast<const T*>(nullptr), 0, partials, st);
-            PM_LAUNCH_CHECK();
-            std::swap(r_in, r_out);
-        }
+        const PcgState* st = queue_pcg<T>(ws, A, b, x, static_cast<const T*>(nullptr), 0, mode, 0.0, 0.0, iterations,
+                                          false, stream);
         fixed_finish_kernel<<<1, 1, 0, stream>>>(st, state->residuals);
         PM_LAUNCH_CHECK();
         PM_CUDA(cudaEventRecord(state->event, stream));
@@ -1433,6 +2189,7 @@ int pm_solver_workspace_close(pm_solver_workspace* ws)
             pm::fail(PM_INVALID_ARGUMENT, "workspace is null");
         ws->drop_graphs(); // they hold pointers into the buffer released here
         ws->buffer.release();
+        ws->mail.buffer.release();
     });
 }
 
