@@ -20,6 +20,7 @@
 //      mode an FP64 iterative-refinement loop around an FP32 inner PCG
 //   5. back-substitution dl = Hll^-1 (-g_l - sum W^T dp)                (thread per block)
 #include "pm_schur.cuh"
+#include "pm_grid.cuh"
 
 #include <algorithm>
 #include <limits>
@@ -60,7 +61,10 @@ struct SolveState // device-side PCG / refinement scalars
     unsigned int ticket[4];
     // stagnation watch: every `window` iterations the residual norm must have halved
     double window_squared;
-    int window, window_start, stagnated, pad2;
+    int window, window_start, stagnated;
+    int timed_out; // one-launch PCG: a grid barrier gave up
+    int checked;   // one-launch PCG: true_squared and rhs_squared are the final step's
+    int pad2;
 };
 
 } // namespace
@@ -72,6 +76,7 @@ struct pm_schur_workspace
     pm::DeviceBuffer numeric;
     pm::DeviceBuffer scratch;
     pm::DeviceBuffer dense; // dense backend: n x n factor and status
+    pm::GridMail mail;      // one-launch PCG
     pm_sparse_workspace* prim_sort = nullptr;
     int64_t pattern_builds = 0;
     const pm_normal_equations* last_ne = nullptr;
@@ -152,6 +157,7 @@ struct pm_schur_workspace
         numeric.release();
         scratch.release();
         dense.release();
+        mail.buffer.release();
         pair_buffer.release();
         if (prim_sort)
             pm_sparse_workspace_destroy(prim_sort);
@@ -1195,7 +1201,7 @@ __device__ __forceinline__ void finish_reduce(double (&mine)[K], double* partial
 // y_p = sum_b S_b x_col(b) for block row p; lane-strided over the row's blocks, warp reduce
 template <typename V, typename M, int BP>
 __device__ __forceinline__ void bsr_row(const int* __restrict__ row_ptr, const int* __restrict__ block_col,
-                                        const M* __restrict__ S, const V* __restrict__ x, int bp_rt, int64_t p,
+                                        const M* __restrict__ S, const V* x, int bp_rt, int64_t p,
                                         bool valid, int lane, double* y /* [16] */)
 {
     constexpr int MP = BP > 0 ? BP : 16;
@@ -1569,6 +1575,200 @@ __global__ void __launch_bounds__(kVecBlock) pcg_block_init_kernel(int64_t P, in
     });
 }
 
+// The whole block-Jacobi PCG in one cooperative launch, a warp per 6x6 block row: lanes 0-5 keep the
+// row's entries of x, r, z and p in registers, the row's preconditioner block is in shared memory,
+// and only p goes through memory for the gathers.  Three grid barriers per iteration (p.q; r.z and
+// r.r; p written) take the place of three kernels, and the kernel goes on to the FP64 true residual
+// of the step it found.  A graph of kernels costs about 10 us an iteration, and a launch, a read and a
+// launch around it, however small the system is.  Solve phase, graph against one launch: 20 block
+// rows, 8 iterations, 167 against 68 us; 501 nearly dense rows in FP32, 4 iterations, 189 against
+// 113; 4,000 rows of 79 blocks, 5 iterations, 254 against 195 (there S is read from HBM).  The
+// arithmetic of every entry is that of the kernels above.
+constexpr int kLoopRows = 32; // warps (block rows) of a CTA, at most
+template <typename V, typename M, typename PM>
+struct SchurLoop
+{
+    int64_t P;
+    const int* row_ptr;
+    const int* block_col;
+    const M* S;
+    const PM* minv;
+    const double* rhs;
+    V* x;
+    V* p;
+    double rel, abs_tol;
+    int rule, max_iterations, window;
+    int x_is_zero; // the initial guess is zero: S x is not formed
+    int check;     // form the true residual of a converged solve (V double)
+    const SchurStatus* status; // factorisations to have succeeded, or null
+    int64_t observations;
+    Packet* mail;
+    unsigned long long epoch;
+    SolveState* st;
+};
+
+__device__ __forceinline__ bool schur_status_bad(const SchurStatus* s, int64_t observations)
+{
+    return s->eliminated_bad != kNone || s->preconditioner_bad != kNone ||
+           (s->observation_bad >= 0 && s->observation_bad < observations);
+}
+
+template <typename V, typename M, typename PM>
+__global__ void __launch_bounds__(32 * kLoopRows, 1) schur_pcg_kernel(const SchurLoop<V, M, PM> a)
+{
+    __shared__ GridShared shared;
+    __shared__ PM blocks[kLoopRows][36];
+    if (a.status && schur_status_bad(a.status, a.observations))
+        return; // nothing is solved; the host reports why
+    SolveState* const st = a.st;
+    GridSync sync{a.mail, &st->timed_out, &shared, a.epoch};
+    if (threadIdx.x == 0)
+        shared.failed = 0; // read after the first barrier's __syncthreads
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t row = int64_t(blockIdx.x) * (blockDim.x >> 5) + warp;
+    const bool valid = row < a.P, own = valid && lane < 6;
+    const int64_t i = row * 6 + lane;
+    const bool writer = blockIdx.x == 0 && threadIdx.x == 0;
+    if (valid)
+        for (int k = lane; k < 36; k += 32)
+            blocks[warp][k] = a.minv[row * 36 + k];
+    __syncwarp();
+    // entry `lane` of S times the vector v (lanes 0-5)
+    auto product = [&](const V* v) {
+        double out[16], y = 0.0;
+        bsr_row<V, M, 6>(a.row_ptr, a.block_col, a.S, v, 6, row, valid, lane, out);
+#pragma unroll
+        for (int k = 0; k < 6; ++k)
+            y = lane == k ? out[k] : y;
+        return y;
+    };
+    // entry `lane` of the preconditioner block times r
+    auto precondition = [&](double r) {
+        double s = 0.0;
+#pragma unroll
+        for (int c = 0; c < 6; ++c)
+        {
+            const double rc = __shfl_sync(0xffffffffu, r, c);
+            s += static_cast<double>(blocks[warp][(lane < 6 ? lane : 0) * 6 + c]) * rc;
+        }
+        return static_cast<double>(static_cast<V>(s));
+    };
+    const double b = own ? a.rhs[i] : 0.0;
+    double x = own && !a.x_is_zero ? static_cast<double>(a.x[i]) : 0.0;
+    double r, z, p;
+    {
+        double q = 0.0;
+        if (!a.x_is_zero)
+            q = static_cast<double>(static_cast<V>(product(a.x)));
+        r = own ? static_cast<double>(static_cast<V>(b - q)) : 0.0;
+    }
+    z = precondition(r);
+    if (own)
+        a.p[i] = static_cast<V>(z);
+    p = z;
+    double mine[2] = {own ? r * z : 0.0, own ? r * r : 0.0}, total[2];
+    if (!grid_sum<2>(sync, mine, total, true))
+        return;
+    double rho = total[0], residual = total[1], window_squared = residual;
+    const double initial = residual, r0 = sqrt(fmax(0.0, residual));
+    const double tolerance = a.rule == 0 ? a.abs_tol + a.rel * r0 : fmax(a.abs_tol, a.rel * r0);
+    int iterations = 0, window_start = 0, converged = 0, breakdown = 0, stagnated = 0;
+    bool done = a.max_iterations <= 0;
+    if (!isfinite(residual))
+    {
+        breakdown = 1;
+        done = true;
+    }
+    else if (r0 <= tolerance)
+    {
+        converged = 1;
+        done = true;
+    }
+    while (!done)
+    {
+        const double q = static_cast<double>(static_cast<V>(product(a.p)));
+        double pq[1] = {own ? p * q : 0.0}, den[1];
+        if (!grid_sum<1>(sync, pq, den, false))
+            return;
+        if (!(den[0] > 0.0) || !isfinite(den[0]))
+        {
+            breakdown = 1;
+            break;
+        }
+        const double alpha = rho / den[0];
+        x = static_cast<double>(static_cast<V>(x + alpha * p));
+        r = own ? static_cast<double>(static_cast<V>(r - alpha * q)) : 0.0;
+        z = precondition(r);
+        mine[0] = own ? r * z : 0.0;
+        mine[1] = own ? r * r : 0.0;
+        if (!grid_sum<2>(sync, mine, total, false))
+            return;
+        iterations += 1;
+        residual = total[1];
+        if (!isfinite(residual))
+        {
+            breakdown = 1;
+            break;
+        }
+        if (sqrt(fmax(0.0, residual)) <= tolerance)
+        {
+            converged = 1;
+            break;
+        }
+        if (iterations >= a.max_iterations)
+            break;
+        if (a.window > 0 && iterations - window_start >= a.window)
+        {
+            if (residual > 0.25 * window_squared) // the norm did not halve over the window
+            {
+                stagnated = 1;
+                break;
+            }
+            window_start = iterations;
+            window_squared = residual;
+        }
+        const double beta = total[0] / rho;
+        rho = total[0];
+        p = static_cast<double>(static_cast<V>(z + beta * p));
+        if (own)
+            a.p[i] = static_cast<V>(p);
+        if (!grid_barrier(sync))
+            return;
+    }
+    if (own)
+        a.x[i] = static_cast<V>(x);
+    bool checked = false;
+    if (a.check && converged)
+    {
+        if (!grid_barrier(sync))
+            return;
+        const double q = product(a.x);
+        const double v = own ? b - q : 0.0;
+        mine[0] = v * v;
+        mine[1] = b * b;
+        if (!grid_sum<2>(sync, mine, total, false))
+            return;
+        checked = true;
+    }
+    if (writer)
+    {
+        st->tolerance = tolerance;
+        st->initial_squared = initial;
+        st->residual_squared = residual;
+        st->iterations = iterations;
+        st->converged = converged;
+        st->breakdown = breakdown;
+        st->stagnated = stagnated;
+        st->done = 1;
+        if (checked)
+        {
+            st->true_squared = total[0];
+            st->rhs_squared = total[1];
+            st->checked = 1;
+        }
+    }
+}
+
 // FP64 residual of the refinement loop: r = b - q (q = S64 x), ||r||^2, ||b||^2
 __global__ void __launch_bounds__(kVecBlock) residual_kernel(int64_t n, const double* __restrict__ b,
                                                              const double* __restrict__ q, double* __restrict__ r,
@@ -1736,8 +1936,11 @@ template <typename T, int BP, int BL>
 __global__ void backsub_kernel(int64_t L, int bp_rt, int bl_rt, const int* __restrict__ cross_offsets,
                                const int* __restrict__ cross_primary, const T* __restrict__ w,
                                const T* __restrict__ gl, const double* __restrict__ hinv, int hstride,
-                               int factor, const T* __restrict__ dp, T* __restrict__ dl)
+                               int factor, const T* __restrict__ dp, T* __restrict__ dl,
+                               const SolveState* __restrict__ state)
 {
+    if (state && !state->converged) // queued behind a solve that did not converge (or did not run)
+        return;
     constexpr int ML = BL > 0 ? BL : 16;
     const int bp = BP > 0 ? BP : bp_rt;
     const int bl = BL > 0 ? BL : bl_rt;
@@ -2750,13 +2953,61 @@ cudaGraphExec_t pcg_iteration_graph(pm_schur_workspace* ws, const M* S, const PM
     return exec;
 }
 
-// One preconditioned CG solve on the block-CSR operand (matrix M, vectors V, inverses PM): the
-// initial residual, then the iteration graph (the device ends it), then one read of the final
-// state, which is returned.
+// One-launch PCG: 6x6 blocks and a warp of the chip for every block row (4,736 rows)
+inline bool one_launch_pcg(const pm_schur_workspace* ws)
+{
+    return ws->bp == 6 && ws->P > 0 && ws->P <= int64_t(kLoopRows) * std::min(sm_count(), kGridMaxCtas);
+}
+
+// Queues it.  check: the FP64 true residual of the step; status: solve only if the factorisations
+// succeeded and no observation was rejected
+template <typename V, typename M, typename PM>
+void queue_one_launch_pcg(pm_schur_workspace* ws, cudaStream_t stream, const M* S, const PM* minv, const double* rhs,
+                          V* x, double rel, double abs_tol, int rule, int max_iterations, V* scratch, int window,
+                          bool x_is_zero, bool check = false, const SchurStatus* status = nullptr,
+                          int64_t observations = 0)
+{
+    ws->mail.open(stream, "SchurComplementSolverWorkspace");
+    SchurLoop<V, M, PM> a{ws->P, ws->block_row_ptr, ws->block_col, S, minv, rhs, x, scratch, rel, abs_tol, rule,
+                          max_iterations, window, x_is_zero, check, status, observations, ws->mail.packets(),
+                          ws->mail.epoch, ws->state};
+    // one CTA while it holds all rows (its barriers are the cheapest), else the fewest rows per CTA
+    int rows = kLoopRows;
+    if (ws->P > kLoopRows)
+        for (rows = 8; rows < kLoopRows && ws->P > int64_t(rows) * std::min(sm_count(), kGridMaxCtas);)
+            rows *= 2;
+    PM_CUDA(cudaMemsetAsync(ws->state, 0, sizeof(SolveState), stream));
+    void* args[] = {&a};
+    PM_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(schur_pcg_kernel<V, M, PM>),
+                                        dim3(grid_for(ws->P, rows)), dim3(32 * rows), args, 0, stream));
+    PM_LAUNCH_CHECK();
+}
+
+// the device state, read after everything queued so far
+SolveState read_solve_state(pm_schur_workspace* ws, cudaStream_t stream)
+{
+    PM_CUDA(cudaMemcpyAsync(ws->host_state, ws->state, sizeof(SolveState), cudaMemcpyDeviceToHost, stream));
+    PM_CUDA(cudaEventRecord(ws->sync_event, stream));
+    PM_CUDA(cudaEventSynchronize(ws->sync_event));
+    if (ws->host_state->timed_out)
+        fail(PM_CUDA_ERROR, "Schur PCG: a grid barrier did not complete");
+    return *ws->host_state;
+}
+
+// One preconditioned CG solve on the block-CSR operand (matrix M, vectors V, inverses PM) and one
+// read of the final state, which is returned: one launch (schur_pcg_kernel) where every block row
+// has a warp, else the initial residual, then the iteration graph (the device ends it).
 template <typename V, typename M, typename PM>
 SolveState block_pcg(pm_schur_workspace* ws, cudaStream_t stream, const M* S, const PM* minv, const double* rhs,
-                     V* x, double rel, double abs_tol, int rule, int max_iterations, V* scratch, int window = 0)
+                     V* x, double rel, double abs_tol, int rule, int max_iterations, V* scratch, int window = 0,
+                     bool x_is_zero = false)
 {
+    if (one_launch_pcg(ws))
+    {
+        queue_one_launch_pcg<V, M, PM>(ws, stream, S, minv, rhs, x, rel, abs_tol, rule, max_iterations, scratch,
+                                       window, x_is_zero);
+        return read_solve_state(ws, stream);
+    }
     const int64_t P = ws->P, n = ws->P * ws->bp;
     const int bp = static_cast<int>(ws->bp);
     V* r0 = scratch;
@@ -2787,9 +3038,7 @@ SolveState block_pcg(pm_schur_workspace* ws, cudaStream_t stream, const M* S, co
         PM_CUDA(cudaMemsetAsync(&ws->state->chunks, 0, sizeof(int), stream));
         PM_CUDA(cudaGraphLaunch(exec, stream));
     }
-    PM_CUDA(cudaMemcpyAsync(ws->host_state, ws->state, sizeof(SolveState), cudaMemcpyDeviceToHost, stream));
-    PM_CUDA(cudaEventRecord(ws->sync_event, stream));
-    PM_CUDA(cudaEventSynchronize(ws->sync_event));
+    read_solve_state(ws, stream);
     if (max_iterations > 0) // the kernels the graph ran: kPcgChunk x 3 + 1 per body
         for (int k = 0; k < ws->host_state->chunks * (3 * kPcgChunk + 1); ++k)
             count_launch();
@@ -3245,10 +3494,50 @@ void schur_solve(pm_schur_workspace* ws, cudaStream_t stream, const pm_normal_eq
         PM_LAUNCH_CHECK();
     }
     PM_CUDA(cudaEventRecord(ws->events[3], stream));
-    // ---- status of the factorisations (one small read; the reference returns early here)
+    // ---- status of the factorisations (one small read; the reference returns early here).  A plain
+    // solve in one launch queues everything first, on the condition of that status, and reads once.
+    double* area = vector_area(ws);
+    const bool queued = !mixed && !dense && !batch && !o->learned && one_launch_pcg(ws);
     PM_CUDA(cudaMemcpyAsync(ws->host_status, ws->status, sizeof(SchurStatus), cudaMemcpyDeviceToHost, stream));
-    PM_CUDA(cudaEventRecord(ws->sync_event, stream));
-    PM_CUDA(cudaEventSynchronize(ws->sync_event));
+    // dl from dp: always, or only if the device state says that the solve converged
+    bool t_at_step = false;
+    auto back_substitute = [&](const SolveState* converged) {
+        if (L <= 0)
+            return;
+        const unsigned grid = grid_for(L, 128, 1 << 20);
+        if (t_at_step && bp == 6 && bl == 3 && sizeof(T) == 8)
+            backsub_from_t_kernel<<<grid, 128, 0, stream>>>(L, ws->hinv, ws->mf_t, reinterpret_cast<double*>(dl));
+        else if (bp == 6 && bl == 3)
+            backsub_kernel<T, 6, 3><<<grid, 128, 0, stream>>>(L, 6, 3, ne->cross_offsets, ne->cross_primary,
+                                                              static_cast<const T*>(ne->cross_values),
+                                                              static_cast<const T*>(ne->eliminated_gradient), ws->hinv,
+                                                              ws->hstride, ws->paired ? 1 : 0, dp, dl, converged);
+        else
+            backsub_kernel<T, 0, 0><<<grid, 128, 0, stream>>>(L, static_cast<int>(bp), static_cast<int>(bl),
+                                                              ne->cross_offsets, ne->cross_primary,
+                                                              static_cast<const T*>(ne->cross_values),
+                                                              static_cast<const T*>(ne->eliminated_gradient), ws->hinv,
+                                                              ws->hstride, 0, dp, dl, converged);
+        PM_LAUNCH_CHECK();
+    };
+    SolveState queued_state{};
+    if (queued)
+    {
+        queue_one_launch_pcg<T, T, double>(ws, stream, static_cast<const T*>(ws->S), ws->minv, ws->rhs, dp,
+                                           o->relative_tolerance, o->absolute_tolerance, o->tolerance_rule,
+                                           o->max_iterations, reinterpret_cast<T*>(area), 0, !o->use_initial_guess,
+                                           o->check_true_residual && sizeof(T) == 8, ws->status,
+                                           ne->observation_status.ptr ? ne->observation_count : 0);
+        PM_CUDA(cudaEventRecord(ws->events[4], stream));
+        back_substitute(ws->state);
+        PM_CUDA(cudaEventRecord(ws->events[5], stream));
+        queued_state = read_solve_state(ws, stream);
+    }
+    else
+    {
+        PM_CUDA(cudaEventRecord(ws->sync_event, stream));
+        PM_CUDA(cudaEventSynchronize(ws->sync_event));
+    }
     ws->assembled = P > 0;
     auto timings = [&](int last) {
         float t = 0.f;
@@ -3335,10 +3624,8 @@ void schur_solve(pm_schur_workspace* ws, cudaStream_t stream, const pm_normal_eq
         }
     };
     // ---- PCG
-    double* area = vector_area(ws);
-    // the FP64 matrix-free pass last run at the final step (mixed precision with FP32 values):
-    // its t_l = Hll^-1 W_l^T dp is the back-substitution's product too
-    bool t_at_step = false;
+    // t_at_step: the FP64 matrix-free pass last run at the final step (mixed precision with FP32
+    // values): its t_l = Hll^-1 W_l^T dp is the back-substitution's product too
     SolveState st{};
     if (n == 0)
     {
@@ -3399,9 +3686,13 @@ void schur_solve(pm_schur_workspace* ws, cudaStream_t stream, const pm_normal_eq
     }
     else if (!mixed)
     {
-        st = block_pcg<T, T, double>(ws, stream, static_cast<const T*>(ws->S), ws->minv, ws->rhs, dp,
-                                     o->relative_tolerance, o->absolute_tolerance, o->tolerance_rule, o->max_iterations,
-                                     reinterpret_cast<T*>(area), learned ? window : 0);
+        if (queued)
+            st = queued_state;
+        else
+            st = block_pcg<T, T, double>(ws, stream, static_cast<const T*>(ws->S), ws->minv, ws->rhs, dp,
+                                         o->relative_tolerance, o->absolute_tolerance, o->tolerance_rule,
+                                         o->max_iterations, reinterpret_cast<T*>(area), learned ? window : 0,
+                                         !o->use_initial_guess);
         rep->initial_residual_norm = std::sqrt(std::max(0.0, st.initial_squared));
         if (learned)
         {
@@ -3464,7 +3755,7 @@ void schur_solve(pm_schur_workspace* ws, cudaStream_t stream, const pm_normal_eq
             // r64 holds b - S x; solve S32 d = r64 to inner_rel (or to the outer target)
             PM_CUDA(cudaMemsetAsync(d32, 0, n * sizeof(float), stream));
             st = block_pcg<float, float, float>(ws, stream, ws->S32, ws->minv32, r64, d32, inner_rel, 0.5 * target, 1,
-                                                o->max_iterations - total, inner, learned ? window : 0);
+                                                o->max_iterations - total, inner, learned ? window : 0, true);
             total += st.iterations;
             rep->refinement_steps += 1;
             if (learned)
@@ -3525,49 +3816,31 @@ void schur_solve(pm_schur_workspace* ws, cudaStream_t stream, const pm_normal_eq
         rep->mixed_precision_used = kept_fp32 ? 1 : 0;
         rep->true_relative_residual = rhs_norm > 0 ? rep->final_residual_norm / rhs_norm : 0.0;
     }
-    PM_CUDA(cudaEventRecord(ws->events[4], stream));
-    if (rep->converged && o->check_true_residual && !mixed && n > 0 && sizeof(T) == 8)
+    if (st.checked)
+        rep->true_relative_residual = st.rhs_squared > 0.0 ? std::sqrt(st.true_squared) / std::sqrt(st.rhs_squared) : 0.0;
+    if (!queued)
     {
-        double* q64 = area + 2 * (n + 1);
-        double norm = 0.0, rhs_norm = 0.0;
-        true_residual<T>(ws, stream, static_cast<const T*>(ws->S), reinterpret_cast<const double*>(dp), q64, nullptr,
-                         norm, rhs_norm);
-        rep->true_relative_residual = rhs_norm > 0 ? norm / rhs_norm : 0.0;
-    }
-    if (!rep->converged)
-    {
+        PM_CUDA(cudaEventRecord(ws->events[4], stream));
+        if (rep->converged && o->check_true_residual && !mixed && n > 0 && sizeof(T) == 8)
+        {
+            double* q64 = area + 2 * (n + 1);
+            double norm = 0.0, rhs_norm = 0.0;
+            true_residual<T>(ws, stream, static_cast<const T*>(ws->S), reinterpret_cast<const double*>(dp), q64, nullptr,
+                             norm, rhs_norm);
+            rep->true_relative_residual = rhs_norm > 0 ? norm / rhs_norm : 0.0;
+        }
+        // ---- back-substitution
+        if (rep->converged)
+            back_substitute(nullptr);
         PM_CUDA(cudaEventRecord(ws->events[5], stream));
         PM_CUDA(cudaEventSynchronize(ws->events[5]));
-        timings(5);
-        note_learned();
-        if (rep->message[0] == '\0')
-            std::snprintf(rep->message, sizeof(rep->message), "PCG iteration limit reached");
-        return;
     }
-    // ---- back-substitution
-    if (L > 0)
-    {
-        const unsigned grid = grid_for(L, 128, 1 << 20);
-        if (t_at_step && bp == 6 && bl == 3 && sizeof(T) == 8)
-            backsub_from_t_kernel<<<grid, 128, 0, stream>>>(L, ws->hinv, ws->mf_t, reinterpret_cast<double*>(dl));
-        else if (bp == 6 && bl == 3)
-            backsub_kernel<T, 6, 3><<<grid, 128, 0, stream>>>(L, 6, 3, ne->cross_offsets, ne->cross_primary,
-                                                              static_cast<const T*>(ne->cross_values),
-                                                              static_cast<const T*>(ne->eliminated_gradient), ws->hinv,
-                                                              ws->hstride, ws->paired ? 1 : 0, dp, dl);
-        else
-            backsub_kernel<T, 0, 0><<<grid, 128, 0, stream>>>(L, static_cast<int>(bp), static_cast<int>(bl),
-                                                              ne->cross_offsets, ne->cross_primary,
-                                                              static_cast<const T*>(ne->cross_values),
-                                                              static_cast<const T*>(ne->eliminated_gradient), ws->hinv,
-                                                              ws->hstride, 0, dp, dl);
-        PM_LAUNCH_CHECK();
-    }
-    PM_CUDA(cudaEventRecord(ws->events[5], stream));
-    PM_CUDA(cudaEventSynchronize(ws->events[5]));
     timings(5);
     note_learned();
-    std::snprintf(rep->message, sizeof(rep->message), "converged");
+    if (rep->converged)
+        std::snprintf(rep->message, sizeof(rep->message), "converged");
+    else if (rep->message[0] == '\0')
+        std::snprintf(rep->message, sizeof(rep->message), "PCG iteration limit reached");
 }
 
 template <typename T, typename O>
