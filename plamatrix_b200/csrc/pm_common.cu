@@ -106,6 +106,30 @@ __global__ void __launch_bounds__(kScanBlock) scan_apply_kernel(const Tin* in, i
         out[n] = running;
 }
 
+// n <= kShortScan: one launch, an element per thread.  Every CTA sums all elements before its own
+// tile, which costs less than the two launches of the levels above (13,824 elements: 4.5 us against
+// 11.5 for three); at most 64 loads a thread.
+constexpr int kShortThreads = 1024;
+constexpr int64_t kShortScan = 64 * kShortThreads;
+template <typename Tin, typename Tout>
+__global__ void __launch_bounds__(kShortThreads) scan_short_kernel(const Tin* __restrict__ in, Tout* __restrict__ out,
+                                                                   int n)
+{
+    __shared__ Tout smem[kShortThreads / 32 + 1];
+    const int base = blockIdx.x * kShortThreads, i = base + threadIdx.x;
+    const Tout mine = i < n ? static_cast<Tout>(in[i]) : Tout(0);
+    Tout before = Tout(0), total;
+#pragma unroll 8
+    for (int k = threadIdx.x; k < base; k += kShortThreads)
+        before += static_cast<Tout>(in[k]);
+    before = block_sum<Tout, kShortThreads>(before, smem);
+    const Tout inside = block_exclusive_scan<Tout, kShortThreads>(mine, smem, total);
+    if (i < n)
+        out[i] = before + inside;
+    if (i == n - 1)
+        out[n] = before + inside + mine;
+}
+
 int64_t tiles_of(int64_t n) { return n <= 0 ? 1 : (n + kScanTile - 1) / kScanTile; }
 
 } // namespace
@@ -132,6 +156,13 @@ void exclusive_scan(const Tin* in, Tout* out, int64_t n, void* scratch, cudaStre
     if (tiles <= 1)
     {
         scan_apply_kernel<Tin, Tout><<<1, kScanBlock, 0, stream>>>(in, n, nullptr, out);
+        PM_LAUNCH_CHECK();
+        return;
+    }
+    if (n <= kShortScan)
+    {
+        scan_short_kernel<Tin, Tout><<<static_cast<unsigned>((n + kShortThreads - 1) / kShortThreads), kShortThreads, 0,
+                                       stream>>>(in, out, static_cast<int>(n));
         PM_LAUNCH_CHECK();
         return;
     }

@@ -240,10 +240,12 @@ struct CooView
 };
 
 // keep_sorted: store every row's sorted keys and values (coo_view readers need them); a
-// conversion that only fills a CSR passes false, and its fill re-sorts the short rows
+// conversion that only fills a CSR passes false, and its fill re-sorts the short rows; filled: a fill
+// that ends the status is queued behind it
 template <typename T>
 void coo_prepare(pm_sparse_workspace* ws, cudaStream_t stream, int64_t rows, int64_t cols, int64_t count,
-                 const int64_t* row_indices, const int64_t* col_indices, const T* values, bool keep_sorted = true);
+                 const int64_t* row_indices, const int64_t* col_indices, const T* values, bool keep_sorted = true,
+                 bool filled = false);
 CooView coo_view(const pm_sparse_workspace* ws);
 int64_t coo_internal_status(pm_sparse_workspace* ws, cudaStream_t stream, const char* operation);
 
@@ -261,6 +263,10 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src)
 __device__ __forceinline__ void cp_async8(void* dst, const void* src)
 {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async4(void* dst, const void* src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(smem_addr(dst)), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 // wait until at most N of this thread's committed groups are still in flight
