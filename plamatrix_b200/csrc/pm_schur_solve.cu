@@ -103,6 +103,7 @@ struct pm_schur_workspace
     int64_t U = 0;
     int2* pairs = nullptr;         // E: {row-list entry of cross (l, p), row-list entry of cross (l, q)}, per block in ascending l
     void* vfactor = nullptr;       // C x 18 (Scalar): V = W_lp L_l^-T of every row-list entry (written by the diagonal pass)
+    bool shape_pinned = false;     // the caller or the autotuner chose upper_shape
     int upper_shape = 0;           // launch shape of the upper-block pass (index into kUpperShapes)
     int* saved_offsets = nullptr;
     int* saved_primary = nullptr;
@@ -1116,26 +1117,61 @@ __global__ void __launch_bounds__(kUpperThreads, SPLIT == 4 ? 3 : 2) assemble_up
 }
 
 // Block-Jacobi preconditioner of the assembled system: FP64 inverse of every diagonal block
-// (symmetrised from its lower triangle), thread per block row.
+// (symmetrised from its lower triangle), BP threads per block row.  Each factors the block and solves
+// for its own column, with the arithmetic of spd_inverse: a thread doing all columns is a chain of 93
+// divisions and square roots, this one of 33 (the assembly phase 2.66 -> 2.63 ms with 4,000 rows, 40 ->
+// 32 us with 20).
 template <typename T, int BP>
 __global__ void diag_inverse_kernel(int64_t P, const int* __restrict__ diag_pos, const T* __restrict__ S,
                                     double* __restrict__ minv, SchurStatus* status)
 {
-    for (int64_t p = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; p < P; p += int64_t(gridDim.x) * blockDim.x)
+    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < P * BP; i += int64_t(gridDim.x) * blockDim.x)
     {
+        const int64_t p = i / BP;
+        const int col = static_cast<int>(i - p * BP);
         const T* d = S + int64_t(diag_pos[p]) * BP * BP;
-        double m[BP * BP], inv[BP * BP], lower[BP * BP], work[BP];
+        double lower[BP][BP], x[BP];
+        bool good = true;
+#pragma unroll
         for (int r = 0; r < BP; ++r)
-            for (int c = 0; c < BP; ++c)
-                m[r * BP + c] = static_cast<double>(r >= c ? d[r * BP + c] : d[c * BP + r]);
-        if (!spd_inverse<BP>(m, BP, inv, lower, work))
+#pragma unroll
+            for (int c = 0; c <= r; ++c)
+            {
+                double value = static_cast<double>(d[r * BP + c]);
+#pragma unroll
+                for (int k = 0; k < c; ++k)
+                    value = __dadd_rn(value, -__dmul_rn(lower[r][k], lower[c][k]));
+                if (r == c)
+                {
+                    good = good && value > 0.0 && isfinite(value);
+                    lower[r][r] = sqrt(value);
+                }
+                else
+                    lower[r][c] = value / lower[c][c];
+            }
+#pragma unroll
+        for (int r = 0; r < BP; ++r)
         {
-            atomicMin(&status->preconditioner_bad, static_cast<long long>(p));
-            for (int k = 0; k < BP * BP; ++k)
-                inv[k] = 0.0;
+            double value = r == col ? 1.0 : 0.0;
+#pragma unroll
+            for (int k = 0; k < r; ++k)
+                value = __dadd_rn(value, -__dmul_rn(lower[r][k], x[k]));
+            x[r] = value / lower[r][r];
         }
-        for (int k = 0; k < BP * BP; ++k)
-            minv[p * BP * BP + k] = inv[k];
+#pragma unroll
+        for (int r = BP - 1; r >= 0; --r)
+        {
+            double value = x[r];
+#pragma unroll
+            for (int k = r + 1; k < BP; ++k)
+                value = __dadd_rn(value, -__dmul_rn(lower[k][r], x[k]));
+            x[r] = value / lower[r][r];
+        }
+        if (!good && col == 0)
+            atomicMin(&status->preconditioner_bad, static_cast<long long>(p));
+#pragma unroll
+        for (int r = 0; r < BP; ++r)
+            minv[p * BP * BP + r * BP + col] = good ? x[r] : 0.0;
     }
 }
 
@@ -1789,50 +1825,138 @@ __global__ void __launch_bounds__(kVecBlock) residual_kernel(int64_t n, const do
     });
 }
 
+// W_l^T x of 32 eliminated blocks per warp, FP64 6x3 cross blocks.  The blocks' crosses are one
+// contiguous run; the warp takes them 32 at a time, a lane per cross: the rows come into shared memory
+// by coalesced asynchronous copies one step ahead (a 144-byte stride is free of bank conflicts for
+// 16-byte reads), x by primary index two steps after the index.  A lane reading its own block's rows
+// takes a line per 16 bytes: 15 load wavefronts per cross and half of the lanes idle (2 + Poisson(4)
+// crosses), 0.49 ms for 12M crosses with the load pipe 77% busy; here about 7 and 0.43 ms.  The products of a
+// cross are summed by row and the crosses of a block in their order, as before.
+// fold(l of this lane, v[3]) is called once per cross of the lane's eliminated block, in cross order.
+constexpr int kRunWarps = 4;
+struct CrossRun // of one warp
+{
+    double w[2][32][18];
+    double u[32][3];
+};
+
+template <bool X16, typename Product, typename Fold>
+__device__ __forceinline__ void cross_run(CrossRun& run, int lo, int hi, int cb, int ce,
+                                          const int* __restrict__ cross_primary, const double* __restrict__ w,
+                                          const double* __restrict__ x, Product&& product, Fold&& fold)
+{
+    const int lane = threadIdx.x & 31;
+    auto stage = [&](int c0, int buffer) { // crosses c0 .. c0 + 31, those before ce
+        const int pieces = min(32, ce - c0) * 9;
+        const double* const src = w + int64_t(c0) * 18;
+        double* const dst = &run.w[buffer][0][0];
+#pragma unroll
+        for (int k = 0; k < 9; ++k)
+            if (k * 32 + lane < pieces)
+                cp_async16(dst + (k * 32 + lane) * 2, src + (k * 32 + lane) * 2);
+        cp_async_commit();
+    };
+    auto gather = [&](int primary, double (&v)[6]) {
+        // x is the caller's vector: pairs when it starts on a 16-byte boundary (checked by the host)
+        const double* const at = x + int64_t(primary) * 6;
+        if constexpr (X16)
+            load_pairs<double, 6>(at, v);
+        else
+#pragma unroll
+            for (int r = 0; r < 6; ++r)
+                v[r] = __ldg(at + r);
+    };
+    int primary = cb + lane < ce ? cross_primary[cb + lane] : 0;
+    int primary_next = cb + 32 + lane < ce ? cross_primary[cb + 32 + lane] : 0;
+    double xv[6], xn[6];
+    if (cb < ce)
+        stage(cb, 0);
+    gather(primary, xv);
+    int buffer = 0;
+    for (int c0 = cb; c0 < ce; c0 += 32, buffer ^= 1)
+    {
+        if (c0 + 32 < ce)
+        {
+            stage(c0 + 32, buffer ^ 1);
+            gather(primary_next, xn);
+            primary_next = c0 + 64 + lane < ce ? cross_primary[c0 + 64 + lane] : 0;
+            cp_async_wait<1>();
+        }
+        else
+            cp_async_wait<0>();
+        __syncwarp();
+        if (c0 + lane < ce)
+        {
+            double wv[18], v[3];
+            const double2* const row = reinterpret_cast<const double2*>(run.w[buffer][lane]);
+#pragma unroll
+            for (int k = 0; k < 9; ++k)
+            {
+                const double2 a = row[k];
+                wv[2 * k] = a.x;
+                wv[2 * k + 1] = a.y;
+            }
+            product(wv, xv, v);
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+                run.u[lane][k] = v[k];
+        }
+        __syncwarp();
+        for (int c = max(lo, c0); c < min(hi, c0 + 32); ++c)
+            fold(run.u[c - c0]);
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < 6; ++k)
+            xv[k] = xn[k];
+    }
+}
+
 // FP64 matrix-free product q = S x of the damped 6x3 Schur complement, straight from the FP64
 // normal equations (used when the assembled values are FP32 only):
 //   q_p = (Hpp_p + damping) x_p + sum_q C_pq x_q - sum_{l in p} W_lp Hll^-1 sum_{q in l} W_lq^T x_q
-// where C are the primary-primary coupling blocks.  Pass 1, thread per eliminated block:
+// where C are the primary-primary coupling blocks.  Pass 1, 32 eliminated blocks per warp:
 // t_l = Hll^-1 (W_l^T x) = L^-T (L^-1 W_l^T x) from the factor record; pass 2, CTA per block row:
 // the row's crosses in row-list order, then a fixed xor tree and the warps in order.  Both passes
 // sum in fixed orders, so the product repeats bit for bit.
-template <typename T, bool X16>
-__global__ void mf_eliminated6_kernel(int64_t L, const int* __restrict__ cross_offsets,
-                                      const int* __restrict__ cross_primary, const T* __restrict__ w,
-                                      const double* __restrict__ rec, const double* __restrict__ x,
-                                      double* __restrict__ t)
+template <bool X16>
+__global__ void __launch_bounds__(32 * kRunWarps) mf_eliminated6_kernel(int64_t L, const int* __restrict__ cross_offsets,
+                                                                        const int* __restrict__ cross_primary,
+                                                                        const double* __restrict__ w,
+                                                                        const double* __restrict__ rec,
+                                                                        const double* __restrict__ x,
+                                                                        double* __restrict__ t)
 {
-    for (int64_t l = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; l < L; l += int64_t(gridDim.x) * blockDim.x)
-    {
-        double u0 = 0.0, u1 = 0.0, u2 = 0.0;
-        for (int c = cross_offsets[l]; c < cross_offsets[l + 1]; ++c)
-        {
-            double wv[18], xv[6];
-            load_pairs<T, 18>(w + int64_t(c) * 18, wv);
-            // x is the caller's step vector: pairs when it starts on a 16-byte boundary (X16,
-            // checked by the host), element by element otherwise
-            const double* xp = x + int64_t(cross_primary[c]) * 6;
-            if constexpr (X16)
-                load_pairs<double, 6>(xp, xv);
-            else
-#pragma unroll
-                for (int r = 0; r < 6; ++r)
-                    xv[r] = xp[r];
+    __shared__ __align__(16) CrossRun runs[kRunWarps];
+    const int lane = threadIdx.x & 31;
+    const int64_t l0 = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) & ~int64_t(31), l = l0 + lane;
+    if (l0 >= L)
+        return;
+    const int lo = cross_offsets[min(l, L)], hi = cross_offsets[min(l + 1, L)];
+    double u[3] = {0.0, 0.0, 0.0};
+    cross_run<X16>(
+        runs[threadIdx.x >> 5], lo, hi, __shfl_sync(0xffffffffu, lo, 0), __shfl_sync(0xffffffffu, hi, 31), cross_primary,
+        w, x,
+        [](const double (&wv)[18], const double (&xv)[6], double (&v)[3]) {
+            v[0] = v[1] = v[2] = 0.0;
 #pragma unroll
             for (int r = 0; r < 6; ++r)
-            {
-                u0 += wv[3 * r] * xv[r];
-                u1 += wv[3 * r + 1] * xv[r];
-                u2 += wv[3 * r + 2] * xv[r];
-            }
-        }
-        double f[10];
-        load_pairs<double, 10>(rec + l * 10, f);
-        const double v0 = f[0] * u0, v1 = f[1] * u0 + f[2] * u1, v2 = f[3] * u0 + f[4] * u1 + f[5] * u2;
-        double2* out = reinterpret_cast<double2*>(t + l * 4);
-        out[0] = make_double2(f[0] * v0 + f[1] * v1 + f[3] * v2, f[2] * v1 + f[4] * v2);
-        out[1] = make_double2(f[5] * v2, 0.0);
-    }
+#pragma unroll
+                for (int c = 0; c < 3; ++c)
+                    v[c] += wv[3 * r + c] * xv[r];
+        },
+        [&](const double (&v)[3]) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+                u[c] += v[c];
+        });
+    if (l >= L)
+        return;
+    double f[10];
+    load_pairs<double, 10>(rec + l * 10, f);
+    const double v0 = f[0] * u[0], v1 = f[1] * u[0] + f[2] * u[1], v2 = f[3] * u[0] + f[4] * u[1] + f[5] * u[2];
+    double2* out = reinterpret_cast<double2*>(t + l * 4);
+    out[0] = make_double2(f[0] * v0 + f[1] * v1 + f[3] * v2, f[2] * v1 + f[4] * v2);
+    out[1] = make_double2(f[5] * v2, 0.0);
 }
 
 template <typename T>
@@ -1932,6 +2056,59 @@ __global__ void backsub_from_t_kernel(int64_t L, const double* __restrict__ rec,
     }
 }
 
+// the same from the cross blocks (FP64 6x3, factor records)
+template <bool X16>
+__global__ void __launch_bounds__(32 * kRunWarps) backsub6_kernel(int64_t L, const int* __restrict__ cross_offsets,
+                                                                  const int* __restrict__ cross_primary,
+                                                                  const double* __restrict__ w,
+                                                                  const double* __restrict__ gl,
+                                                                  const double* __restrict__ rec,
+                                                                  const double* __restrict__ dp,
+                                                                  double* __restrict__ dl,
+                                                                  const SolveState* __restrict__ state)
+{
+    if (state && !state->converged) // queued behind a solve that did not converge (or did not run)
+        return;
+    __shared__ __align__(16) CrossRun runs[kRunWarps];
+    const int lane = threadIdx.x & 31;
+    const int64_t l0 = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) & ~int64_t(31), l = l0 + lane;
+    if (l0 >= L)
+        return;
+    const int lo = cross_offsets[min(l, L)], hi = cross_offsets[min(l + 1, L)];
+    double u[3] = {0.0, 0.0, 0.0};
+    if (l < L)
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+            u[c] = -gl[l * 3 + c];
+    cross_run<X16>(
+        runs[threadIdx.x >> 5], lo, hi, __shfl_sync(0xffffffffu, lo, 0), __shfl_sync(0xffffffffu, hi, 31), cross_primary,
+        w, dp,
+        [](const double (&wv)[18], const double (&xv)[6], double (&v)[3]) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+            {
+                v[c] = 0.0;
+#pragma unroll
+                for (int r = 0; r < 6; ++r)
+                    v[c] = __dadd_rn(v[c], __dmul_rn(wv[3 * r + c], xv[r]));
+            }
+        },
+        [&](const double (&v)[3]) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+                u[c] = __dadd_rn(u[c], -v[c]);
+        });
+    if (l >= L)
+        return;
+    double f[10];
+    load_pairs<double, 10>(rec + l * 10, f);
+    // Hll^-1 u = L^-T (L^-1 u) from the factor record [L^-1 00, 10, 11, 20, 21, 22 | z]
+    const double v0 = f[0] * u[0], v1 = f[1] * u[0] + f[2] * u[1], v2 = f[3] * u[0] + f[4] * u[1] + f[5] * u[2];
+    dl[l * 3] = f[0] * v0 + f[1] * v1 + f[3] * v2;
+    dl[l * 3 + 1] = f[2] * v1 + f[4] * v2;
+    dl[l * 3 + 2] = f[5] * v2;
+}
+
 template <typename T, int BP, int BL>
 __global__ void backsub_kernel(int64_t L, int bp_rt, int bl_rt, const int* __restrict__ cross_offsets,
                                const int* __restrict__ cross_primary, const T* __restrict__ w,
@@ -1953,41 +2130,12 @@ __global__ void backsub_kernel(int64_t L, int bp_rt, int bl_rt, const int* __res
         {
             const T* W = w + int64_t(c) * bp * bl;
             const T* x = dp + int64_t(cross_primary[c]) * bp;
-            if constexpr (BP == 6 && BL == 3 && sizeof(T) == 8)
+            for (int col = 0; col < bl; ++col)
             {
-                // the cross block as 16-byte loads (the normal-equation buffers are 256-byte aligned
-                // and a block is 144 bytes); the caller's step vector element by element
-                double wv[18], xv[6];
-                const double2* w2 = reinterpret_cast<const double2*>(W);
-#pragma unroll
-                for (int k = 0; k < 9; ++k)
-                {
-                    const double2 a = __ldg(w2 + k);
-                    wv[2 * k] = a.x;
-                    wv[2 * k + 1] = a.y;
-                }
-#pragma unroll
-                for (int k = 0; k < 6; ++k)
-                    xv[k] = static_cast<double>(x[k]);
-#pragma unroll
-                for (int col = 0; col < 3; ++col)
-                {
-                    double v = 0.0;
-#pragma unroll
-                    for (int row = 0; row < 6; ++row)
-                        v = __dadd_rn(v, __dmul_rn(wv[row * 3 + col], xv[row]));
-                    point[col] = add_rn(point[col], static_cast<T>(-v));
-                }
-            }
-            else
-            {
-                for (int col = 0; col < bl; ++col)
-                {
-                    T v = T(0);
-                    for (int row = 0; row < bp; ++row)
-                        v = add_rn(v, mul_rn(W[row * bl + col], x[row]));
-                    point[col] = add_rn(point[col], -v);
-                }
+                T v = T(0);
+                for (int row = 0; row < bp; ++row)
+                    v = add_rn(v, mul_rn(W[row * bl + col], x[row]));
+                point[col] = add_rn(point[col], -v);
             }
         }
         const double* H = hinv + l * hstride;
@@ -2389,6 +2537,23 @@ struct UpperShape
 constexpr UpperShape kUpperShapes[] = {{8, 2}, {4, 2}, {16, 2}, {4, 4}, {8, 4}, {2, 2}, {1, 2}};
 constexpr int kUpperShapeCount = sizeof(kUpperShapes) / sizeof(kUpperShapes[0]);
 
+// The shape of a workspace whose caller chose none, by pairs per upper block, number of upper blocks
+// and type of the V rows.  Measured assembly, us, for (8,2) (4,2) (4,4) (8,4):
+//   few pairs per block leave streams idle: 3.0 pairs, 118,140 blocks, FP32 134 99 97 146; 4.2 pairs,
+//     2.1M blocks, FP64 2772 2345 2520 3132; 54.6 pairs, 155,726 blocks, FP64 775 728 755 800;
+//   many pairs want all eight: 217.8 pairs, 156,000 blocks, FP64 2642 2671 2716 2660; 174 pairs, 11,700
+//     blocks, FP64 243 277 246 227;
+//   four lanes a pair keep 24 instead of 16 warps per SM, which pays with FP32 rows (217.8 pairs, FP32
+//     1935 1972 1851 1859) and with fewer blocks (27 pairs, 19,900 blocks, FP64 113 113 103 113);
+//   below some 4,000 blocks a block's own chain is all there is: 63 pairs, 190 blocks, FP64 37 43 44 37.
+int default_shape(const pm_schur_workspace* ws, bool fp64)
+{
+    const bool split2 = fp64 && ws->U >= 65536;
+    if (ws->E < 64 * ws->U && ws->U >= 4096)
+        return split2 ? 1 : 3;
+    return split2 ? 0 : 4;
+}
+
 template <typename TO, typename TP, typename VT, typename AT, int STREAMS, int SPLIT>
 void launch_upper_shape(pm_schur_workspace* ws, const int* block_pc, const VT* vf, const TP* pcv, TO* S,
                         cudaStream_t stream)
@@ -2403,7 +2568,7 @@ template <typename TO, typename TP, typename VT, typename AT>
 void launch_upper(pm_schur_workspace* ws, const int* block_pc, const VT* vf, const TP* pcv, TO* S,
                   cudaStream_t stream)
 {
-    switch (ws->upper_shape)
+    switch (ws->shape_pinned ? ws->upper_shape : default_shape(ws, sizeof(VT) == 8))
     {
     case 1: launch_upper_shape<TO, TP, VT, AT, 4, 2>(ws, block_pc, vf, pcv, S, stream); break;
     case 2: launch_upper_shape<TO, TP, VT, AT, 16, 2>(ws, block_pc, vf, pcv, S, stream); break;
@@ -2478,7 +2643,7 @@ void launch_assembly(pm_schur_workspace* ws, const pm_normal_equations* ne, doub
             launch_upper<T, T, T, double>(ws, a.block_pc, vf, a.pcv, a.S, stream);
         }
         ws->s32_only = fp32_products;
-        diag_inverse_kernel<T, 6><<<grid_for(a.P, 64, 1 << 16), 64, 0, stream>>>(a.P, a.diag_pos, a.S, a.minv,
+        diag_inverse_kernel<T, 6><<<grid_for(a.P * 6, 64, 1 << 16), 64, 0, stream>>>(a.P, a.diag_pos, a.S, a.minv,
                                                                                  a.status);
         PM_LAUNCH_CHECK();
     }
@@ -3062,13 +3227,13 @@ void true_residual(pm_schur_workspace* ws, cudaStream_t stream, const M* S, cons
     {
         // the assembled values are FP32: the FP64 product comes from the FP64 normal equations
         const pm_normal_equations* ne = ws->last_ne;
-        const unsigned egrid = grid_for(ws->L, 128, 1 << 20);
+        const unsigned egrid = grid_for(ws->L, 32 * kRunWarps);
         if (reinterpret_cast<uintptr_t>(x) % 16 == 0)
-            mf_eliminated6_kernel<double, true><<<egrid, 128, 0, stream>>>(
+            mf_eliminated6_kernel<true><<<egrid, 32 * kRunWarps, 0, stream>>>(
                 ws->L, ne->cross_offsets, ne->cross_primary, static_cast<const double*>(ne->cross_values), ws->hinv,
                 x, ws->mf_t);
         else
-            mf_eliminated6_kernel<double, false><<<egrid, 128, 0, stream>>>(
+            mf_eliminated6_kernel<false><<<egrid, 32 * kRunWarps, 0, stream>>>(
                 ws->L, ne->cross_offsets, ne->cross_primary, static_cast<const double*>(ne->cross_values), ws->hinv,
                 x, ws->mf_t);
         PM_LAUNCH_CHECK();
@@ -3507,6 +3672,19 @@ void schur_solve(pm_schur_workspace* ws, cudaStream_t stream, const pm_normal_eq
         const unsigned grid = grid_for(L, 128, 1 << 20);
         if (t_at_step && bp == 6 && bl == 3 && sizeof(T) == 8)
             backsub_from_t_kernel<<<grid, 128, 0, stream>>>(L, ws->hinv, ws->mf_t, reinterpret_cast<double*>(dl));
+        else if (ws->paired && sizeof(T) == 8)
+        {
+            const auto run = [&](auto kernel) {
+                kernel<<<grid_for(L, 32 * kRunWarps), 32 * kRunWarps, 0, stream>>>(
+                    L, ne->cross_offsets, ne->cross_primary, static_cast<const double*>(ne->cross_values),
+                    static_cast<const double*>(ne->eliminated_gradient), ws->hinv,
+                    reinterpret_cast<const double*>(dp), reinterpret_cast<double*>(dl), converged);
+            };
+            if (reinterpret_cast<uintptr_t>(dp) % 16 == 0)
+                run(backsub6_kernel<true>);
+            else
+                run(backsub6_kernel<false>);
+        }
         else if (bp == 6 && bl == 3)
             backsub_kernel<T, 6, 3><<<grid, 128, 0, stream>>>(L, 6, 3, ne->cross_offsets, ne->cross_primary,
                                                               static_cast<const T*>(ne->cross_values),
@@ -3585,7 +3763,7 @@ void schur_solve(pm_schur_workspace* ws, cudaStream_t stream, const pm_normal_eq
     bool learned = o->learned && bp == 6 && n > 0;
     const int window = o->stagnation_window > 0 ? o->stagnation_window : 25;
     auto restore_block_jacobi = [&]() {
-        diag_inverse_kernel<T, 6><<<grid_for(P, 64, 1 << 16), 64, 0, stream>>>(P, ws->diag_pos,
+        diag_inverse_kernel<T, 6><<<grid_for(P * 6, 64, 1 << 16), 64, 0, stream>>>(P, ws->diag_pos,
                                                                                 static_cast<const T*>(ws->S),
                                                                                 ws->minv, ws->status);
         PM_LAUNCH_CHECK();
@@ -3899,6 +4077,7 @@ void autotune_assembly(pm_schur_workspace* ws, cudaStream_t stream, const pm_nor
     for (int k = 0; k < kUpperShapeCount; ++k)
     {
         ws->upper_shape = k;
+        ws->shape_pinned = true;
         launch_assembly<T>(ws, ne, ws->damping, ws->min_diag, stream, fp32); // warm-up
         PM_CUDA(cudaEventRecord(e0, stream));
         for (int r = 0; r < repeats; ++r)
@@ -3982,6 +4161,7 @@ int pm_schur_set_assembly_shape(pm_schur_workspace* ws, int shape)
         if (shape < 0 || shape >= pm::kUpperShapeCount)
             pm::fail(PM_INVALID_ARGUMENT, "assembly shape out of range");
         ws->upper_shape = shape;
+        ws->shape_pinned = true;
     });
 }
 
