@@ -111,3 +111,23 @@ def test_default_shape_and_inverses(P, L, k, precision):
         inverse = torch.linalg.inv(blocks)
         got = s["preconditioner"].view(P, 6, 6)
         assert ((got - inverse).flatten(1).norm(dim=1) <= 1e-10 * inverse.flatten(1).norm(dim=1)).all()
+
+
+def test_batched_graph_follows_the_batch():
+    """One workspace over batches of other sizes, options and step vectors: its kept iteration graph
+    gives the bits of a fresh workspace every time."""
+    batches = [[(12, 700), (30, 900)], [(40, 2000), (9, 500), (25, 800)], [(12, 700), (30, 900)]]
+    shared = SC.SchurComplementSolverWorkspace()
+    for k, sizes in enumerate(batches):
+        probs = [W.bundle_problem(P, L, per_eliminated=4, seed=10 * k + i) for i, (P, L) in enumerate(sizes)]
+        union = SC.pack_observation_systems(probs)
+        ne = _equations(union)
+        for precision, tol in (("native", 1e-8), ("native", 1e-6), ("mixed", 1e-8), ("native", 1e-8)):
+            opts = SC.SchurComplementSolverOptions(max_iterations=200, relative_tolerance=tol, precision=precision)
+            hold = torch.empty(6 * union["P"] + 64, dtype=torch.float64, device="cuda")  # moves the next step vector
+            got = SC.solve_batched_schur_complement(ne, 1e-3, union["primary_offsets"], opts, shared)
+            want = SC.solve_batched_schur_complement(ne, 1e-3, union["primary_offsets"], opts)
+            assert got[2]["converged"] and want[2]["converged"]
+            assert [s["iterations"] for s in got[3]] == [s["iterations"] for s in want[3]]
+            assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+            del hold
