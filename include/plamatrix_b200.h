@@ -404,7 +404,8 @@ PM_API int pm_schur_solve_f64(pm_schur_workspace* workspace, pm_stream_t stream,
  * block_schur_device_assembly.cu:211-220).  The upper-block pass of the 6x3 assembly has
  * pm_schur_assembly_shape_count() lane layouts ({pair streams, lanes per pair}); each sums every
  * block in a fixed order of its own, so a shape gives repeatable values, and shapes differ from
- * one another only by rounding.  pm_schur_autotune_assembly times every shape `repeats` times on
+ * one another only by rounding.  A workspace whose caller sets none takes the shape from the system's
+ * pairs per block, block count and type.  pm_schur_autotune_assembly times every shape `repeats` times on
  * the system `workspace` last solved (`equations` must be that system), keeps the fastest in the
  * workspace and reports its index, its mean ms and (shape_ms_h, may be NULL, one per shape)
  * every shape's mean ms.  It reassembles the system, so the workspace needs a new solve before

@@ -15,10 +15,10 @@
 //      masks (integer atomicOr: order independent), then the thread owning a block walks its
 //      mask in cross order and accumulates the 6x6 product in registers.  No float atomics:
 //      the result is bitwise reproducible.  Lower blocks are mirrored afterwards.
-//   4. block-Jacobi PCG on the 6x6 block-CSR (warp per block row SpMV with 128-bit loads,
-//      FP64 dots finished by the last block, alpha/beta/convergence on the device); in mixed
-//      mode an FP64 iterative-refinement loop around an FP32 inner PCG
-//   5. back-substitution dl = Hll^-1 (-g_l - sum W^T dp)                (thread per block)
+//   4. block-Jacobi PCG on the 6x6 block-CSR (warp per block row with 128-bit loads, FP64 dots,
+//      alpha/beta/convergence on the device): one cooperative launch up to 4,736 block rows, else
+//      a graph of kernels; in mixed mode an FP64 iterative-refinement loop around an FP32 inner PCG
+//   5. back-substitution dl = Hll^-1 (-g_l - sum W^T dp)                (32 blocks per warp)
 #include "pm_schur.cuh"
 #include "pm_grid.cuh"
 
