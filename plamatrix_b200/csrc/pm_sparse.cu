@@ -15,6 +15,7 @@
 //     when the solve is done and the host reads the state once, after it.
 #include "pm_common.cuh"
 #include "pm_grid.cuh"
+#include "pm_piece.h"
 
 #include <cmath>
 #include <limits>
@@ -98,7 +99,8 @@ __global__ void validate_csr_kernel(int64_t rows, int64_t cols, int64_t nnz, con
 // row of A x with a TPR-wide sub-warp per row; x_at(c) is entry c of x; G of a lane's nonzeros are
 // loaded at a time: columns and values, then the gathers, all in flight together.  A row of 474 on 32
 // lanes waits for two rounds of loads with G = 8 instead of 15 (24,000 rows: FP32 16.6 -> 15.1 us, FP64
-// 33.0 -> 27.0 us, L2 warm).
+// 33.0 -> 27.0 us, L2 warm).  Positions go up to 2^31 - 3, so loops count what is left of a row: a
+// position a stride past its end would not fit in an int.
 template <typename T, int TPR, int G, typename Gather>
 __device__ __forceinline__ T csr_row_dot(const int* __restrict__ rp, const int* __restrict__ ci,
                                          const T* __restrict__ v, Gather&& x_at, int64_t row, bool valid, int lane)
@@ -107,52 +109,28 @@ __device__ __forceinline__ T csr_row_dot(const int* __restrict__ rp, const int* 
     if (valid)
     {
         const int b = rp[row], e = rp[row + 1];
-        if constexpr (TPR == 1)
+        const int* c = ci + b + lane;
+        const T* w = v + b + lane;
+        for (int left = e - b - lane; left > 0; left -= G * TPR, c += G * TPR, w += G * TPR)
         {
-            // a thread per row: streamed, no reuse, the sum in storage order
-            for (int base = b; base < e; base += G)
-            {
-                int col[G];
-                T val[G], xv[G];
+            int col[G];
+            T val[G], xv[G];
 #pragma unroll
-                for (int k = 0; k < G; ++k)
-                    if (base + k < e)
-                    {
-                        col[k] = __ldcs(ci + base + k);
-                        val[k] = __ldcs(v + base + k);
-                    }
+            for (int k = 0; k < G; ++k)
+                if (k * TPR < left)
+                {
+                    // a thread per row: streamed, no reuse
+                    col[k] = TPR == 1 ? __ldcs(c + k * TPR) : c[k * TPR];
+                    val[k] = TPR == 1 ? __ldcs(w + k * TPR) : w[k * TPR];
+                }
 #pragma unroll
-                for (int k = 0; k < G; ++k)
-                    if (base + k < e)
-                        xv[k] = x_at(col[k]);
+            for (int k = 0; k < G; ++k)
+                if (k * TPR < left)
+                    xv[k] = x_at(col[k]);
 #pragma unroll
-                for (int k = 0; k < G; ++k)
-                    if (base + k < e)
-                        sum += val[k] * xv[k];
-            }
-        }
-        else
-        {
-            for (int p = b + lane; p < e; p += G * TPR)
-            {
-                int col[G];
-                T val[G], xv[G];
-#pragma unroll
-                for (int k = 0; k < G; ++k)
-                    if (p + k * TPR < e)
-                    {
-                        col[k] = ci[p + k * TPR];
-                        val[k] = v[p + k * TPR];
-                    }
-#pragma unroll
-                for (int k = 0; k < G; ++k)
-                    if (p + k * TPR < e)
-                        xv[k] = x_at(col[k]);
-#pragma unroll
-                for (int k = 0; k < G; ++k)
-                    if (p + k * TPR < e)
-                        sum += val[k] * xv[k];
-            }
+            for (int k = 0; k < G; ++k)
+                if (k * TPR < left)
+                    sum += val[k] * xv[k];
         }
     }
 #pragma unroll
@@ -205,15 +183,14 @@ __device__ __forceinline__ void tile_load(RowTile<T, CAP>& tile, const int* __re
     {
         const int k = (u * 32 + lane) * 4;
         if (k < count)
-            cp_async16_stream(tile.col + k, ci + first + k, min(16, (nnz - first - k) * 4), policy);
+            cp_async16_stream(tile.col + k, ci + first + k, piece_bytes(nnz - first - k, sizeof(int)), policy);
     }
 #pragma unroll
     for (int u = 0; u < (CAP + 32 * kPer - 1) / (32 * kPer); ++u)
     {
         const int k = (u * 32 + lane) * kPer;
         if (k < count)
-            cp_async16_stream(tile.val + k, v + first + k,
-                              min(16, (nnz - first - k) * static_cast<int>(sizeof(T))), policy);
+            cp_async16_stream(tile.val + k, v + first + k, piece_bytes(nnz - first - k, sizeof(T)), policy);
     }
 }
 
@@ -245,10 +222,11 @@ __device__ __forceinline__ T tile_row(RowTile<T, CAP>& tile, const int* __restri
                                       Gather&& x_at)
 {
     T sum = tile_sum(tile, b - first, min(e - first, CAP), T(0), x_at);
-    for (int at = first + CAP; at < end; at += CAP)
+    for (int left = end - first - CAP; left > 0; left -= CAP)
     {
+        const int at = end - left;
         __syncwarp();
-        tile_load(tile, ci, v, at, min(end - at, CAP), nnz, policy, lane);
+        tile_load(tile, ci, v, at, min(left, CAP), nnz, policy, lane);
         cp_async_commit();
         cp_async_wait<0>();
         __syncwarp();
@@ -561,21 +539,22 @@ __device__ __forceinline__ void jacobi_row(int64_t r, const int* __restrict__ rp
     double diag = 0.0, scale = 0.0;
     bool found = false;
     constexpr int G = 8; // loads in flight
-    const int e = rp[r + 1];
-    for (int p = rp[r]; p < e; p += G)
+    const int* c = ci + rp[r];
+    const T* w = v + rp[r];
+    for (int left = rp[r + 1] - rp[r]; left > 0; left -= G, c += G, w += G)
     {
         int col[G];
         T value[G];
 #pragma unroll
         for (int k = 0; k < G; ++k)
-            if (p + k < e)
+            if (k < left)
             {
-                col[k] = ci[p + k];
-                value[k] = v[p + k];
+                col[k] = c[k];
+                value[k] = w[k];
             }
 #pragma unroll
         for (int k = 0; k < G; ++k)
-            if (p + k < e)
+            if (k < left)
             {
                 scale = fmax(scale, fabs(static_cast<double>(value[k])));
                 if (col[k] == r)
