@@ -2099,6 +2099,8 @@ void pm_csr_destroy(pm_csr* A)
 {
     if (A)
     {
+        // stream-ordered memory: cudaFree does not wait for the kernels that still read it
+        cudaDeviceSynchronize();
         cudaFree(A->row_ptr);
         cudaFree(A->col_idx);
         delete A;
