@@ -1,0 +1,36 @@
+"""Schur solves at the limits of the problem's shape."""
+import numpy as np
+import pytest
+import torch
+
+from gpu_util import host
+from plamatrix_b200 import schur as SC
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("L", [1, 32, 70])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_no_primary_blocks(L, dtype):
+    """P = 0: every eliminated block is moved by its own damped gradient, and the empty primary step is
+    neither read nor written.  The 3x3 systems have condition numbers below 100: 1e-12 (FP64) and 1e-4
+    (FP32) relative are far above their rounding."""
+    rng = np.random.default_rng(L)
+    a = rng.standard_normal((L, 3, 3))
+    hessian = (a @ a.transpose(0, 2, 1) + 3.0 * np.eye(3)).astype(dtype)
+    gradient = rng.standard_normal((L, 3)).astype(dtype)
+    ne = SC.DeviceNormalEquations(0, L, 6, 3, dtype)
+    ne.upload({"primary_diagonal": np.zeros((0, 6, 6)), "eliminated_diagonal": hessian,
+               "primary_gradient": np.zeros((0, 6)), "eliminated_gradient": gradient,
+               "adjacency_offsets": np.zeros(L + 1, np.int64), "cross_primary": np.zeros(0, np.int64),
+               "cross_values": np.zeros((0, 6, 3)), "primary_cross_row": np.zeros(0, np.int64),
+               "primary_cross_col": np.zeros(0, np.int64), "primary_cross_values": np.zeros((0, 6, 6))})
+    step = torch.empty(0, dtype=ne.tdtype, device="cuda")
+    dp, dl, rep = SC.solve_damped_schur_complement(ne, 1e-3, primary_step=step)
+    assert rep["converged"] and rep["iterations"] == 0 and dp.numel() == 0
+    damped = hessian.astype(np.float64).copy()
+    damped[:, range(3), range(3)] *= 1.0 + 1e-3
+    want = np.linalg.solve(damped, -gradient.astype(np.float64)[:, :, None])[:, :, 0]
+    tolerance = 1e-12 if dtype == np.float64 else 1e-4
+    error = np.linalg.norm(host(dl).reshape(-1, 3) - want, axis=1)
+    assert np.all(error <= tolerance * np.linalg.norm(want, axis=1))
