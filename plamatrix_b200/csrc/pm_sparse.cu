@@ -96,11 +96,9 @@ __global__ void validate_csr_kernel(int64_t rows, int64_t cols, int64_t nnz, con
     }
 }
 
-// row of A x with a TPR-wide sub-warp per row; x_at(c) is entry c of x; G of a lane's nonzeros are
-// loaded at a time: columns and values, then the gathers, all in flight together.  A row of 474 on 32
-// lanes waits for two rounds of loads with G = 8 instead of 15 (24,000 rows: FP32 16.6 -> 15.1 us, FP64
-// 33.0 -> 27.0 us, L2 warm).  Positions go up to 2^31 - 3, so loops count what is left of a row: a
-// position a stride past its end would not fit in an int.
+// row of A x with a TPR-wide sub-warp per row; x_at(c) is entry c of x; G > 0 of a lane's nonzeros are
+// loaded at a time: columns and values, then the gathers, all in flight together; 0: one after the other,
+// as the compiler unrolls them (see long_rows).  The order of a lane's sum is the same.
 template <typename T, int TPR, int G, typename Gather>
 __device__ __forceinline__ T csr_row_dot(const int* __restrict__ rp, const int* __restrict__ ci,
                                          const T* __restrict__ v, Gather&& x_at, int64_t row, bool valid, int lane)
@@ -109,28 +107,34 @@ __device__ __forceinline__ T csr_row_dot(const int* __restrict__ rp, const int* 
     if (valid)
     {
         const int b = rp[row], e = rp[row + 1];
-        const int* c = ci + b + lane;
-        const T* w = v + b + lane;
-        for (int left = e - b - lane; left > 0; left -= G * TPR, c += G * TPR, w += G * TPR)
+        if constexpr (G == 0)
         {
-            int col[G];
-            T val[G], xv[G];
+            for (int p = b + lane; p < e; p += TPR)
+                sum += v[p] * x_at(ci[p]);
+        }
+        else
+        {
+            for (int p = b + lane; p < e; p += G * TPR)
+            {
+                int col[G];
+                T val[G], xv[G];
 #pragma unroll
-            for (int k = 0; k < G; ++k)
-                if (k * TPR < left)
-                {
-                    // a thread per row: streamed, no reuse
-                    col[k] = TPR == 1 ? __ldcs(c + k * TPR) : c[k * TPR];
-                    val[k] = TPR == 1 ? __ldcs(w + k * TPR) : w[k * TPR];
-                }
+                for (int k = 0; k < G; ++k)
+                    if (p + k * TPR < e)
+                    {
+                        // a thread per row: streamed, no reuse
+                        col[k] = TPR == 1 ? __ldcs(ci + p + k * TPR) : ci[p + k * TPR];
+                        val[k] = TPR == 1 ? __ldcs(v + p + k * TPR) : v[p + k * TPR];
+                    }
 #pragma unroll
-            for (int k = 0; k < G; ++k)
-                if (k * TPR < left)
-                    xv[k] = x_at(col[k]);
+                for (int k = 0; k < G; ++k)
+                    if (p + k * TPR < e)
+                        xv[k] = x_at(col[k]);
 #pragma unroll
-            for (int k = 0; k < G; ++k)
-                if (k * TPR < left)
-                    sum += val[k] * xv[k];
+                for (int k = 0; k < G; ++k)
+                    if (p + k * TPR < e)
+                        sum += val[k] * xv[k];
+            }
         }
     }
 #pragma unroll
@@ -222,11 +226,12 @@ __device__ __forceinline__ T tile_row(RowTile<T, CAP>& tile, const int* __restri
                                       Gather&& x_at)
 {
     T sum = tile_sum(tile, b - first, min(e - first, CAP), T(0), x_at);
-    for (int left = end - first - CAP; left > 0; left -= CAP)
+    // unsigned: the step past the last piece need not fit in an int
+    for (unsigned next = static_cast<unsigned>(first) + CAP; next < static_cast<unsigned>(end); next += CAP)
     {
-        const int at = end - left;
+        const int at = static_cast<int>(next);
         __syncwarp();
-        tile_load(tile, ci, v, at, min(left, CAP), nnz, policy, lane);
+        tile_load(tile, ci, v, at, min(end - at, CAP), nnz, policy, lane);
         cp_async_commit();
         cp_async_wait<0>();
         __syncwarp();
@@ -366,7 +371,7 @@ __global__ void __launch_bounds__(256) csr_stream_kernel(int64_t rows, const int
     }
 }
 
-template <typename T, int TPR>
+template <typename T, int TPR, int G>
 __global__ void __launch_bounds__(256) csr_spmv_kernel(int64_t rows, const int* __restrict__ rp,
                                                        const int* __restrict__ ci, const T* __restrict__ v,
                                                        const T* __restrict__ x, T* __restrict__ y)
@@ -381,7 +386,7 @@ __global__ void __launch_bounds__(256) csr_spmv_kernel(int64_t rows, const int* 
         const int64_t row = first + k * stride;
         const bool valid = row < rows;
         const T sum =
-            csr_row_dot<T, TPR, 8>(rp, ci, v, [&](int c) { return __ldg(x + c); }, row, valid, lane);
+            csr_row_dot<T, TPR, G>(rp, ci, v, [&](int c) { return __ldg(x + c); }, row, valid, lane);
         if (valid && lane == 0)
             y[row] = sum;
     }
@@ -401,6 +406,16 @@ int pick_tpr(int64_t rows, int64_t nnz)
     return tpr;
 }
 
+// Rows of fourteen or more nonzeros per lane, on 32 lanes, are read eight of a lane's at a time (two rounds of
+// loads for a row of 474 instead of fifteen, at 48-64 registers instead of 32): 24,000 rows of 474, L2 warm,
+// FP32 22.7 -> 16.5 us, FP64 50.6 -> 28.9; 12,000 of 1,000, FP32 25.0 -> 16.5, FP64 57.5 -> 28.8.  Below that
+// most of a round is empty and half the warps are gone: 24,000 rows of 400, 30 FP32 iterations 833 us one
+// after the other against 880; 240,000 rows of 32, FP64 57 us against 97; an 80^3 27-point grid 112 against 213.
+inline bool long_rows(const pm_csr* A)
+{
+    return lanes_per_row(A) == 32 && A->nnz >= 14 * 32 * A->rows &&
+           A->nnz <= INT32_MAX - 8 * 32; // positions a round past the end fit in an int
+}
 
 // one lane per row from staged tiles: the values (the caller's array) on a 16-byte boundary
 template <typename T>
@@ -435,12 +450,17 @@ void launch_spmv(const pm_csr* A, const T* x, T* y, cudaStream_t stream)
     const unsigned grid = grid_for(A->rows * lanes_per_row(A), block, 65535);
     switch (lanes_per_row(A))
     {
-    case 1: csr_spmv_kernel<T, 1><<<grid, block, 0, stream>>>(A->rows, A->row_ptr, A->col_idx, v, x, y); break;
-    case 2: csr_spmv_kernel<T, 2><<<grid, block, 0, stream>>>(A->rows, A->row_ptr, A->col_idx, v, x, y); break;
-    case 4: csr_spmv_kernel<T, 4><<<grid, block, 0, stream>>>(A->rows, A->row_ptr, A->col_idx, v, x, y); break;
-    case 8: csr_spmv_kernel<T, 8><<<grid, block, 0, stream>>>(A->rows, A->row_ptr, A->col_idx, v, x, y); break;
-    case 16: csr_spmv_kernel<T, 16><<<grid, block, 0, stream>>>(A->rows, A->row_ptr, A->col_idx, v, x, y); break;
-    default: csr_spmv_kernel<T, 32><<<grid, block, 0, stream>>>(A->rows, A->row_ptr, A->col_idx, v, x, y); break;
+    case 1: csr_spmv_kernel<T, 1, 8><<<grid, block, 0, stream>>>(A->rows, A->row_ptr, A->col_idx, v, x, y); break;
+    case 2: csr_spmv_kernel<T, 2, 0><<<grid, block, 0, stream>>>(A->rows, A->row_ptr, A->col_idx, v, x, y); break;
+    case 4: csr_spmv_kernel<T, 4, 0><<<grid, block, 0, stream>>>(A->rows, A->row_ptr, A->col_idx, v, x, y); break;
+    case 8: csr_spmv_kernel<T, 8, 0><<<grid, block, 0, stream>>>(A->rows, A->row_ptr, A->col_idx, v, x, y); break;
+    case 16: csr_spmv_kernel<T, 16, 0><<<grid, block, 0, stream>>>(A->rows, A->row_ptr, A->col_idx, v, x, y); break;
+    default:
+        if (long_rows(A))
+            csr_spmv_kernel<T, 32, 8><<<grid, block, 0, stream>>>(A->rows, A->row_ptr, A->col_idx, v, x, y);
+        else
+            csr_spmv_kernel<T, 32, 0><<<grid, block, 0, stream>>>(A->rows, A->row_ptr, A->col_idx, v, x, y);
+        break;
     }
     PM_LAUNCH_CHECK();
 }
@@ -1146,7 +1166,7 @@ __device__ __forceinline__ void pcg_step(PcgState* st, double den, T)
 }
 
 // q = A p, alpha = rho / p.q
-template <typename T, int TPR>
+template <typename T, int TPR, int G>
 __global__ void __launch_bounds__(kReduceBlock) pcg_spmv_kernel(int64_t rows, const int* __restrict__ rp,
                                                                 const int* __restrict__ ci, const T* __restrict__ v,
                                                                 const T* __restrict__ p, T* __restrict__ q,
@@ -1163,7 +1183,7 @@ __global__ void __launch_bounds__(kReduceBlock) pcg_spmv_kernel(int64_t rows, co
     {
         const int64_t row = first + k * stride;
         const bool valid = row < rows;
-        const T sum = csr_row_dot<T, TPR, 8>(rp, ci, v, [&](int c) { return __ldg(p + c); }, row, valid, lane);
+        const T sum = csr_row_dot<T, TPR, G>(rp, ci, v, [&](int c) { return __ldg(p + c); }, row, valid, lane);
         if (valid && lane == 0)
         {
             q[row] = sum;
@@ -1677,12 +1697,19 @@ void launch_pcg_spmv(const pm_csr* A, const T* p, T* q, double* partials, PcgSta
     }
     switch (lanes_per_row(A))
     {
-    case 1: pcg_spmv_kernel<T, 1><<<grid, kReduceBlock, 0, stream>>>(A->rows, A->row_ptr, A->col_idx, v, p, q, partials, st); break;
-    case 2: pcg_spmv_kernel<T, 2><<<grid, kReduceBlock, 0, stream>>>(A->rows, A->row_ptr, A->col_idx, v, p, q, partials, st); break;
-    case 4: pcg_spmv_kernel<T, 4><<<grid, kReduceBlock, 0, stream>>>(A->rows, A->row_ptr, A->col_idx, v, p, q, partials, st); break;
-    case 8: pcg_spmv_kernel<T, 8><<<grid, kReduceBlock, 0, stream>>>(A->rows, A->row_ptr, A->col_idx, v, p, q, partials, st); break;
-    case 16: pcg_spmv_kernel<T, 16><<<grid, kReduceBlock, 0, stream>>>(A->rows, A->row_ptr, A->col_idx, v, p, q, partials, st); break;
-    default: pcg_spmv_kernel<T, 32><<<grid, kReduceBlock, 0, stream>>>(A->rows, A->row_ptr, A->col_idx, v, p, q, partials, st); break;
+    case 1: pcg_spmv_kernel<T, 1, 8><<<grid, kReduceBlock, 0, stream>>>(A->rows, A->row_ptr, A->col_idx, v, p, q, partials, st); break;
+    case 2: pcg_spmv_kernel<T, 2, 0><<<grid, kReduceBlock, 0, stream>>>(A->rows, A->row_ptr, A->col_idx, v, p, q, partials, st); break;
+    case 4: pcg_spmv_kernel<T, 4, 0><<<grid, kReduceBlock, 0, stream>>>(A->rows, A->row_ptr, A->col_idx, v, p, q, partials, st); break;
+    case 8: pcg_spmv_kernel<T, 8, 0><<<grid, kReduceBlock, 0, stream>>>(A->rows, A->row_ptr, A->col_idx, v, p, q, partials, st); break;
+    case 16: pcg_spmv_kernel<T, 16, 0><<<grid, kReduceBlock, 0, stream>>>(A->rows, A->row_ptr, A->col_idx, v, p, q, partials, st); break;
+    default:
+        if (long_rows(A))
+            pcg_spmv_kernel<T, 32, 8><<<grid, kReduceBlock, 0, stream>>>(A->rows, A->row_ptr, A->col_idx, v, p, q,
+                                                                          partials, st);
+        else
+            pcg_spmv_kernel<T, 32, 0><<<grid, kReduceBlock, 0, stream>>>(A->rows, A->row_ptr, A->col_idx, v, p, q,
+                                                                          partials, st);
+        break;
     }
     PM_LAUNCH_CHECK();
 }

@@ -1,0 +1,87 @@
+"""SpMV and the solvers where the choice of a row kernel changes.
+
+Tolerances: SpMV within the summation-order bound (row length + 1) eps sum |a_ij x_j|.  The matrices are
+strictly diagonally dominant with a condition number below 30: a solution of an FP64 solve to 1e-10 is within
+1e-8 of the reference's, an FP32 one (1e-6, vectors rounded to FP32) within 1e-4."""
+import numpy as np
+import pytest
+import torch
+
+from gpu_util import dev, host, tdtype
+from plamatrix_b200 import sparse as S
+
+pytestmark = pytest.mark.gpu
+
+
+def _symmetric(lengths, seed):
+    """A symmetric matrix whose rows have about `lengths` nonzeros: a diagonal of twice the absolute sum of
+    the rest of the row, and wrapped bands whose reach follows the length."""
+    rng = np.random.default_rng(seed)
+    n = len(lengths)
+    reach = (np.asarray(lengths) - 1) // 2
+    i = np.repeat(np.arange(n), reach)
+    step = np.concatenate([np.arange(1, k + 1) for k in reach]) if len(i) else np.zeros(0, np.int64)
+    j = (i + step) % n
+    keep = i != j
+    i, j = i[keep], j[keep]
+    v = rng.uniform(-1.0, 1.0, len(i))
+    weight = np.zeros(n)
+    np.add.at(weight, i, np.abs(v))
+    np.add.at(weight, j, np.abs(v))
+    r, c = np.concatenate([np.arange(n), i, j]), np.concatenate([np.arange(n), j, i])
+    v = np.concatenate([2.0 * weight + 1.0, v, v])
+    order = np.lexsort((c, r))
+    offsets = np.zeros(n + 1, np.int64)
+    np.cumsum(np.bincount(r, minlength=n), out=offsets[1:])
+    return offsets, c[order].astype(np.int64), v[order]
+
+
+def _operand(matrix, dtype):
+    ro, ci, v = matrix
+    n = len(ro) - 1
+    return S.CsrOperand(S.CSRMatrix(n, n, dev(ro), dev(ci), dev(v.astype(dtype))))
+
+
+def _check_product(checkers, matrix, dtype):
+    ro, ci, v = matrix
+    n = len(ro) - 1
+    op = _operand(matrix, dtype)
+    x = np.random.default_rng(n).uniform(-1.0, 1.0, n).astype(dtype)
+    want = checkers.csr_spmv(ro, ci, v, x.astype(np.float64))
+    size = checkers.csr_spmv(ro, ci, np.abs(v), np.abs(x.astype(np.float64)))
+    error = np.abs(host(op.spmv(dev(x))).astype(np.float64) - want)
+    assert np.all(error <= (np.diff(ro) + 1) * np.finfo(dtype).eps * size)
+    return op, x
+
+
+def _check(checkers, matrix, dtype, solvers=("pcg",)):
+    ro, ci, v = matrix
+    n = len(ro) - 1
+    v = v.astype(dtype).astype(np.float64)
+    op, x = _check_product(checkers, (ro, ci, v), dtype)
+    solution, report = checkers.pcg(ro, ci, v, x.astype(np.float64), relative_tolerance=1e-12)
+    assert report["converged"]
+    options = S.IterativeSolverOptions(relative_tolerance=1e-10 if dtype == np.float64 else 1e-6)
+    for kind in solvers:
+        got = torch.zeros(n, dtype=tdtype(dtype), device="cuda")
+        more = ()
+        if kind == "block_pcg":  # the inverse diagonal in blocks of three
+            inverse = np.zeros((n // 3, 3, 3))
+            rows = np.repeat(np.arange(n), np.diff(ro))
+            inverse[np.arange(n) // 3, np.arange(n) % 3, np.arange(n) % 3] = 1.0 / v[rows == ci]
+            more = (dev(inverse.reshape(-1).astype(dtype)), 3)
+        report = getattr(S, kind)(op, dev(x), got, *more, options=options)
+        assert report["converged"]
+        tolerance = 1e-8 if dtype == np.float64 else 1e-4
+        assert np.linalg.norm(host(got) - solution) <= tolerance * np.linalg.norm(solution)
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("n", [700, 5000])
+@pytest.mark.parametrize("length", [33, 257, 447, 449, 513, 655])
+def test_long_rows(checkers, dtype, n, length):
+    """Fewer and more than fourteen nonzeros per lane, even and uneven rows, in one launch and as kernels."""
+    even = np.full(n, length)
+    _check(checkers, _symmetric(even, n), dtype, ("pcg", "cg"))
+    uneven = np.random.default_rng(length).integers(length // 2, length + length // 2, n)
+    _check(checkers, _symmetric(uneven, n), dtype)
