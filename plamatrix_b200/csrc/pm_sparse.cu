@@ -146,8 +146,7 @@ __device__ __forceinline__ T csr_row_dot(const int* __restrict__ rp, const int* 
 // ------------------------------------------------------------------ staged row tiles
 // One lane per row with the matrix staged in shared memory.  A warp takes tiles of 32 consecutive
 // rows; the tile's nonzeros are one contiguous range of columns and values, brought in by 16-byte
-// asynchronous copies (coalesced, two tiles in flight per warp, marked evict-first in L2 so that
-// the vectors stay), and lane i then sums row i in storage order from shared memory.  Reading the
+// asynchronous copies (coalesced, marked evict-first in L2 so that the vectors stay), and lane i then sums row i in storage order from shared memory.  Reading the
 // same rows directly costs a lane-strided access per nonzero: 180 load wavefronts per 32 rows of
 // seven FP64 nonzeros against about 100 here, and at 180 the load pipe (45 us for the 128^3
 // Laplacian) is slower than HBM.
@@ -198,11 +197,10 @@ __device__ __forceinline__ void tile_load(RowTile<T, CAP>& tile, const int* __re
     }
 }
 
-// sum + the products of the staged positions [lo, hi), in order; gathers in groups of eight
-template <typename T, int CAP, typename Gather>
+// sum + the products of the staged positions [lo, hi), in order; gathers in groups of G
+template <int G, typename T, int CAP, typename Gather>
 __device__ __forceinline__ T tile_sum(const RowTile<T, CAP>& tile, int lo, int hi, T sum, Gather&& x_at)
 {
-    constexpr int G = 8;
     for (int base = lo; base < hi; base += G)
     {
         T xv[G];
@@ -220,12 +218,12 @@ __device__ __forceinline__ T tile_sum(const RowTile<T, CAP>& tile, int lo, int h
 
 // the row [b, e) of a tile whose nonzeros are [first, end), its first piece staged; tiles longer
 // than the capacity load their other pieces here
-template <typename T, int CAP, typename Gather>
+template <int G, typename T, int CAP, typename Gather>
 __device__ __forceinline__ T tile_row(RowTile<T, CAP>& tile, const int* __restrict__ ci, const T* __restrict__ v,
                                       int b, int e, int first, int end, int nnz, uint64_t policy, int lane,
                                       Gather&& x_at)
 {
-    T sum = tile_sum(tile, b - first, min(e - first, CAP), T(0), x_at);
+    T sum = tile_sum<G>(tile, b - first, min(e - first, CAP), T(0), x_at);
     // unsigned: the step past the last piece need not fit in an int
     for (unsigned next = static_cast<unsigned>(first) + CAP; next < static_cast<unsigned>(end); next += CAP)
     {
@@ -235,14 +233,15 @@ __device__ __forceinline__ T tile_row(RowTile<T, CAP>& tile, const int* __restri
         cp_async_commit();
         cp_async_wait<0>();
         __syncwarp();
-        sum = tile_sum(tile, max(b - at, 0), min(e - at, CAP), sum, x_at);
+        sum = tile_sum<G>(tile, max(b - at, 0), min(e - at, CAP), sum, x_at);
     }
     return sum;
 }
 
 // Every tile warp0, warp0 + warps, ...: done(row, sum) for each of its rows, by the row's lane.
-// Values and columns 16-byte aligned; `stage`: the warp's two tiles.
-template <typename T, int CAP, typename Gather, typename Done>
+// Values and columns 16-byte aligned; `stage`: the warp's tiles, two (the next one is on its way while
+// one is summed) or one.
+template <int BUFFERS, typename T, int CAP, typename Gather, typename Done>
 __device__ __forceinline__ void csr_tiles(RowTile<T, CAP>* stage, int64_t rows, int nnz, const int* __restrict__ rp,
                                           const int* __restrict__ ci, const T* __restrict__ v, int64_t warp0,
                                           int64_t warps, Gather&& x_at, Done&& done)
@@ -268,17 +267,21 @@ __device__ __forceinline__ void csr_tiles(RowTile<T, CAP>* stage, int64_t rows, 
     int b, e, nb, ne, buffer = 0;
     bounds(warp0, b, e);
     bounds(warp0 + warps, nb, ne);
-    issue(stage[0], b, e);
+    if (BUFFERS == 2)
+        issue(stage[0], b, e);
     for (int64_t t = warp0; t < tiles; t += warps)
     {
-        issue(stage[buffer ^ 1], nb, ne);
+        if (BUFFERS == 2)
+            issue(stage[buffer ^ 1], nb, ne);
+        else
+            issue(stage[0], b, e);
         int fb, fe;
         bounds(t + 2 * warps, fb, fe);
-        cp_async_wait<1>();
+        cp_async_wait<BUFFERS - 1>();
         __syncwarp();
         const int first = __shfl_sync(0xffffffffu, b, 0) & ~3;
         const int end = __shfl_sync(0xffffffffu, e, 31);
-        const T sum = tile_row(stage[buffer], ci, v, b, e, first, end, nnz, policy, lane, x_at);
+        const T sum = tile_row<BUFFERS == 1 && sizeof(T) == 4 ? 4 : 8>(stage[buffer], ci, v, b, e, first, end, nnz, policy, lane, x_at);
         if (t * 32 + lane < rows)
             done(t * 32 + lane, sum);
         __syncwarp();
@@ -286,20 +289,33 @@ __device__ __forceinline__ void csr_tiles(RowTile<T, CAP>* stage, int64_t rows, 
         e = ne;
         nb = fb;
         ne = fe;
-        buffer ^= 1;
+        if (BUFFERS == 2)
+            buffer ^= 1;
     }
     cp_async_wait<0>();
 }
 
+// SpMV.  What bounds it is the gathers of x, and the matrix from HBM when it is cold.  One tile of ten
+// nonzeros per row for each warp: a second buffer would take the L1 from the gathers (FP64 197 KB of shared
+// memory an SM against 123) and a capacity of eight per row sends half the tiles of a mean of 7.9 through a
+// second load.  us, directly read / two buffers of 256 / this, L2 warm: 600,000 rows of 7.9 in a random
+// band FP64 24.7 / 33.0 / 22.7, FP32 18.2 / 19.4 / 16.5; 1.5M rows of 7.3 FP64 55.2 / 57.9 / 47.2, FP32
+// 37.0 / 37.1 / 32.7; 128^3 grid FP64 37.0 / 35.0 / 35.0, FP32 26.5 / 28.4 / 26.8, cold FP64 45.1 / 41.0 /
+// 39.0.  Five CTAs per SM and gathers in groups of four in FP32 (48 registers); FP64 spills there.
+constexpr int kSpmvCap = 320;
+constexpr int spmv_ctas(size_t value_size) { return value_size == 8 ? 4 : 5; } // of 256 threads per SM
 template <typename T>
-__global__ void __launch_bounds__(256, 4) csr_tile_kernel(int64_t rows, int nnz, const int* __restrict__ rp,
-                                                          const int* __restrict__ ci, const T* __restrict__ v,
-                                                          const T* __restrict__ x, T* __restrict__ y)
+__global__ void __launch_bounds__(256, spmv_ctas(sizeof(T))) csr_tile_kernel(int64_t rows, int nnz,
+                                                                             const int* __restrict__ rp,
+                                                                             const int* __restrict__ ci,
+                                                                             const T* __restrict__ v,
+                                                                             const T* __restrict__ x,
+                                                                             T* __restrict__ y)
 {
     extern __shared__ __align__(16) unsigned char tile_smem[];
-    csr_tiles(reinterpret_cast<RowTile<T, kTileCap>*>(tile_smem) + 2 * (threadIdx.x >> 5), rows, nnz, rp, ci, v, (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5,
-                 int64_t(gridDim.x) * (blockDim.x >> 5), [&](int c) { return __ldg(x + c); },
-                 [&](int64_t row, T sum) { y[row] = sum; });
+    csr_tiles<1>(reinterpret_cast<RowTile<T, kSpmvCap>*>(tile_smem) + (threadIdx.x >> 5), rows, nnz, rp, ci, v,
+                 (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5, int64_t(gridDim.x) * (blockDim.x >> 5),
+                 [&](int c) { return __ldg(x + c); }, [&](int64_t row, T sum) { y[row] = sum; });
 }
 
 // Row-group stream (chosen by pm_csr_set_kernel or the autotuner): a warp owns 32 consecutive rows.  Their nonzeros form one
@@ -440,9 +456,9 @@ void launch_spmv(const pm_csr* A, const T* x, T* y, cudaStream_t stream)
     }
     if (use_tiles<T>(A))
     {
-        const size_t smem = size_t(block / 32) * 2 * sizeof(RowTile<T, kTileCap>);
+        const size_t smem = size_t(block / 32) * sizeof(RowTile<T, kSpmvCap>);
         allow_smem(reinterpret_cast<const void*>(csr_tile_kernel<T>), smem);
-        csr_tile_kernel<T><<<grid_for(A->rows, block, 4 * sm_count()), block, smem, stream>>>(
+        csr_tile_kernel<T><<<grid_for(A->rows, block, spmv_ctas(sizeof(T)) * sm_count()), block, smem, stream>>>(
             A->rows, static_cast<int>(A->nnz), A->row_ptr, A->col_idx, v, x, y);
         PM_LAUNCH_CHECK();
         return;
@@ -662,7 +678,7 @@ __device__ __forceinline__ void for_rows(const PcgLoop<T>& a, unsigned char* sme
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if constexpr (SHAPE == 1)
     {
-        csr_tiles(reinterpret_cast<RowTile<T, CAP>*>(smem) + 2 * warp, a.n, a.nnz, a.rp, a.ci, a.v, thread >> 5,
+        csr_tiles<2>(reinterpret_cast<RowTile<T, CAP>*>(smem) + 2 * warp, a.n, a.nnz, a.rp, a.ci, a.v, thread >> 5,
                   threads >> 5, x_at, done);
     }
     else if constexpr (SHAPE == 0)
@@ -936,7 +952,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) pcg_row_kernel(const PcgLoop<T
         {
             q[j] = T(0);
             if (staged)
-                q[j] = tile_sum(tile, b[j], e[j], T(0), x_at);
+                q[j] = tile_sum<8>(tile, b[j], e[j], T(0), x_at);
             else
                 for (int k = b[j]; k < e[j]; ++k)
                     q[j] += a.v[k] * x_at(a.ci[k]);
@@ -1233,7 +1249,7 @@ __global__ void __launch_bounds__(kReduceBlock, 4) pcg_tile_spmv_kernel(int64_t 
         return;
     extern __shared__ __align__(16) unsigned char tile_smem[];
     double mine[1] = {0.0};
-    csr_tiles(reinterpret_cast<RowTile<T, kTileCap>*>(tile_smem) + 2 * (threadIdx.x >> 5), rows, nnz, rp, ci, v,
+    csr_tiles<1>(reinterpret_cast<RowTile<T, kSpmvCap>*>(tile_smem) + (threadIdx.x >> 5), rows, nnz, rp, ci, v,
               (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5, int64_t(gridDim.x) * (blockDim.x >> 5),
               [&](int c) { return __ldg(p + c); }, [&](int64_t row, T sum) {
                   q[row] = sum;
@@ -1684,11 +1700,11 @@ void launch_pcg_spmv(const pm_csr* A, const T* p, T* q, double* partials, PcgSta
         PM_LAUNCH_CHECK();
         return;
     }
-    // FP32 only: in FP64 the tiles' 197 KB of shared memory leave the gathers of p too little L1
-    // (150^3: 4.12 ms for 30 iterations against 4.00 read directly; FP32 2.76 against 3.16)
+    // FP32 only: in FP64 a grid's rows are read faster directly (150^3, 30 iterations: 3.87 ms from tiles
+    // against 3.74; FP32 2.60 against 2.93; 600,000 rows of 7.9, blocks of six: FP32 1.19 against 1.30)
     if (sizeof(T) == 4 && use_tiles<T>(A))
     {
-        const size_t smem = size_t(kReduceBlock / 32) * 2 * sizeof(RowTile<T, kTileCap>);
+        const size_t smem = size_t(kReduceBlock / 32) * sizeof(RowTile<T, kSpmvCap>);
         allow_smem(reinterpret_cast<const void*>(pcg_tile_spmv_kernel<T>), smem);
         pcg_tile_spmv_kernel<T><<<std::min<unsigned>(grid, 4 * sm_count()), kReduceBlock, smem, stream>>>(
             A->rows, static_cast<int>(A->nnz), A->row_ptr, A->col_idx, v, p, q, partials, st);

@@ -85,3 +85,32 @@ def test_long_rows(checkers, dtype, n, length):
     _check(checkers, _symmetric(even, n), dtype, ("pcg", "cg"))
     uneven = np.random.default_rng(length).integers(length // 2, length + length // 2, n)
     _check(checkers, _symmetric(uneven, n), dtype)
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("rows", [32, 33, 4800])
+@pytest.mark.parametrize("held", [0, 1, 319, 320, 321, 640, 641, 5000])
+def test_tiles_of_short_rows(checkers, dtype, rows, held):
+    """32 rows of `held` nonzeros among rows of five: a tile below, at and past its capacity of 320, in two
+    pieces and in many, starting at every offset from a 16-byte boundary."""
+    rng = np.random.default_rng(held)
+    for lead in range(4 if rows > 64 else 1):
+        lengths = np.full(rows, 5 if rows > 64 else 0)
+        first = 64 if rows > 64 else 0
+        lengths[0] += lead
+        lengths[first:first + 32] = rng.multinomial(held, np.full(32, 1.0 / 32.0))
+        if rows <= 64 and held > 8 * rows:
+            lengths = np.concatenate([lengths, np.zeros(held // 8 + 1, lengths.dtype)])  # a mean of at most eight
+        offsets = np.zeros(len(lengths) + 1, np.int64)
+        np.cumsum(lengths, out=offsets[1:])
+        columns = rng.integers(0, len(lengths), offsets[-1])
+        values = rng.standard_normal(offsets[-1]).astype(dtype).astype(np.float64)
+        _check_product(checkers, (offsets, columns, values), dtype)
+
+
+@pytest.mark.parametrize("longest", [7, 13])
+def test_tiles_in_the_iteration_graph(checkers, longest):
+    """Block PCG of more rows than one launch holds, FP32: tiles up to and past their capacity."""
+    n = 96_000
+    rows = np.where(np.arange(n) % 640 < 32, longest, 7)
+    _check(checkers, _symmetric(rows, n), np.float32, ("block_pcg",))
