@@ -29,6 +29,7 @@ struct pm_csr
     int* col_idx = nullptr; // int32 copy of the validated column indices
     const void* values = nullptr;
     int threads_per_row = 1; // lanes per row of the heuristic
+    int longest_row = 0;     // its nonzeros
     int kernel = -1;         // -1: heuristic; 0: row-group stream; 1..32: lanes per row (autotuned or set)
 };
 
@@ -65,6 +66,7 @@ struct CsrCheck
     long long bad_column;
     long long bad_value;
     int endpoints_bad;
+    int longest; // nonzeros of a row
 };
 
 template <typename T>
@@ -76,13 +78,18 @@ __global__ void validate_csr_kernel(int64_t rows, int64_t cols, int64_t nnz, con
     const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t == 0 && (row_offsets[0] != 0 || row_offsets[rows] != nnz))
         check->endpoints_bad = 1;
+    int longest = 0;
     for (int64_t r = t; r < rows; r += stride)
     {
         const int64_t b = row_offsets[r], e = row_offsets[r + 1];
         if (b < 0 || e < b || e > nnz)
             atomicMin(&check->bad_offsets_row, static_cast<long long>(r));
         row_ptr32[r] = static_cast<int>(b);
+        longest = static_cast<int>(min(static_cast<int64_t>(INT32_MAX), max(e - b, static_cast<int64_t>(longest))));
     }
+    longest = __reduce_max_sync(0xffffffffu, longest);
+    if (longest > 0 && (threadIdx.x & 31) == 0)
+        atomicMax(&check->longest, longest);
     if (t == 0)
         row_ptr32[rows] = static_cast<int>(nnz);
     for (int64_t p = t; p < nnz; p += stride)
@@ -511,10 +518,11 @@ struct PcgState
 //   pcg_row_kernel   up to 2,048 rows per SM, one lane per row: all vectors in registers, the
 //                    matrix in shared memory (24^3 grid FP32: 5.6 us an iteration against 12.7;
 //                    67^3 FP64: 13.2 against 23.4)
-//   pcg_loop_kernel  KEEP: larger, while the residual fits in shared memory beside the staged tiles
-//                    (128^3 FP64: 67 us an iteration against 79: no z, r out of L2, x and p in one
-//                    pass; DRAM traffic 212 MB an iteration against 308); otherwise systems of few
-//                    lanes in any SpMV shape (360 rows of 360: 9.5 us against 14.5)
+//   pcg_loop_kernel  KEEP: larger, or with a row past kLoneRow, while the residual fits in shared
+//                    memory beside the staged tiles (128^3 FP64: 67 us an iteration against 79: no z,
+//                    r out of L2, x and p in one pass; DRAM traffic 212 MB an iteration against 308);
+//                    otherwise systems of few lanes in any SpMV shape (360 rows of 360: 9.5 us
+//                    against 14.5)
 // Everything else runs the graph: with one CTA of at most 1,024 threads per SM the vector phases
 // of larger systems, and the block preconditioner's, have too few loads in flight (150^3 FP64: 145
 // us an iteration against 132; 24,000 rows of 474 in FP64: 55 against 49).
@@ -1432,7 +1440,7 @@ void csr_create(cudaStream_t stream, int64_t rows, int64_t cols, int64_t nnz, co
         PM_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&A->col_idx), (nnz > 0 ? nnz : 1) * sizeof(int), stream));
         CsrCheck* check = nullptr;
         PM_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&check), sizeof(CsrCheck), stream));
-        CsrCheck init{kNone, kNone, kNone, 0};
+        CsrCheck init{kNone, kNone, kNone, 0, 0};
         PM_CUDA(cudaMemcpyAsync(check, &init, sizeof(init), cudaMemcpyHostToDevice, stream));
         validate_csr_kernel<T><<<grid_for(std::max(rows, nnz), 256, 4096), 256, 0, stream>>>(
             rows, cols, nnz, ro, ci, v, A->row_ptr, A->col_idx, check);
@@ -1461,6 +1469,7 @@ void csr_create(cudaStream_t stream, int64_t rows, int64_t cols, int64_t nnz, co
             m << "CSRMatrix value is not finite at position " << result.bad_value;
             fail(PM_INVALID_ARGUMENT, m.str());
         }
+        A->longest_row = result.longest;
     }
     catch (...)
     {
@@ -1826,14 +1835,22 @@ void launch_cooperative(Kernel kernel, PcgLoop<T>& a, unsigned ctas, unsigned th
 
 // One cooperative launch of the whole solve where it is the faster form (see pcg_loop_kernel);
 // false where it is not.  One CTA per SM at most: they wait for one another, so all must be resident.
+// A lane that sums a longer row alone holds up the whole launch.  Every gathered entry of p formed from two
+// vectors, it takes 103 ns a nonzero in FP64 and 67 in FP32 (36 and 30 from staged tiles, 67 and 65 as kernels
+// that read directly).  Jacobi PCG, 30 iterations, us, as kernels / rows in registers / staged tiles with the
+// kept residual: 60,000 rows of 5 and one of 128, FP64 748 / 600 / 508, FP32 701 / 443 / 452; one of 1,000,
+// 2,555 / 2,753 / 1,214 and 2,104 / 1,711 / 986.  Blocks of six, FP32, one of 1,000: one launch 2,166,
+// kernels 1,437; FP64 1,935 and 2,469.
+constexpr int kLoneRow = 128;
+
 template <typename T, int SHAPE>
-bool launch_pcg_loop_shape(PcgLoop<T>& a, size_t warp_smem, int lanes, cudaStream_t stream)
+bool launch_pcg_loop_shape(PcgLoop<T>& a, size_t warp_smem, int lanes, int longest_row, cudaStream_t stream)
 {
     const int most = std::min(sm_count(), kGridMaxCtas);
     if constexpr (SHAPE == 1)
     {
         constexpr size_t kSmem = 226 * 1024; // of the 227 KB a CTA may have; the rest is static
-        if (a.mode != 2 && a.n <= int64_t(4) * kRowThreads * most)
+        if (a.mode != 2 && a.n <= int64_t(4) * kRowThreads * most && longest_row <= kLoneRow)
         {
             const auto launch_rows = [&](auto kernel, int per_thread) {
                 unsigned block = 256;
@@ -1860,6 +1877,8 @@ bool launch_pcg_loop_shape(PcgLoop<T>& a, size_t warp_smem, int lanes, cudaStrea
         }
         warp_smem = 2 * sizeof(RowTile<T, kTileCap>);
     }
+    if ((SHAPE == -1 || (SHAPE == 1 && sizeof(T) == 4)) && longest_row > kLoneRow)
+        return false;
     // few lanes: one row per thread (or group of lanes)
     constexpr unsigned kMost = loop_threads<T>(SHAPE);
     const int64_t wanted = a.n * lanes;
@@ -1877,17 +1896,17 @@ template <typename T>
 bool launch_pcg_loop(const pm_csr* A, PcgLoop<T>& a, cudaStream_t stream)
 {
     if (use_stream(A))
-        return launch_pcg_loop_shape<T, 0>(a, kStreamCap * sizeof(T), 1, stream);
+        return launch_pcg_loop_shape<T, 0>(a, kStreamCap * sizeof(T), 1, A->longest_row, stream);
     if (use_tiles<T>(A))
-        return launch_pcg_loop_shape<T, 1>(a, 0, 1, stream);
+        return launch_pcg_loop_shape<T, 1>(a, 0, 1, A->longest_row, stream);
     switch (lanes_per_row(A))
     {
-    case 1: return launch_pcg_loop_shape<T, -1>(a, 0, 1, stream);
-    case 2: return launch_pcg_loop_shape<T, 2>(a, 0, 2, stream);
-    case 4: return launch_pcg_loop_shape<T, 4>(a, 0, 4, stream);
-    case 8: return launch_pcg_loop_shape<T, 8>(a, 0, 8, stream);
-    case 16: return launch_pcg_loop_shape<T, 16>(a, 0, 16, stream);
-    default: return launch_pcg_loop_shape<T, 32>(a, 0, 32, stream);
+    case 1: return launch_pcg_loop_shape<T, -1>(a, 0, 1, A->longest_row, stream);
+    case 2: return launch_pcg_loop_shape<T, 2>(a, 0, 2, A->longest_row, stream);
+    case 4: return launch_pcg_loop_shape<T, 4>(a, 0, 4, A->longest_row, stream);
+    case 8: return launch_pcg_loop_shape<T, 8>(a, 0, 8, A->longest_row, stream);
+    case 16: return launch_pcg_loop_shape<T, 16>(a, 0, 16, A->longest_row, stream);
+    default: return launch_pcg_loop_shape<T, 32>(a, 0, 32, A->longest_row, stream);
     }
 }
 

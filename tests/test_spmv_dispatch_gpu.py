@@ -114,3 +114,15 @@ def test_tiles_in_the_iteration_graph(checkers, longest):
     n = 96_000
     rows = np.where(np.arange(n) % 640 < 32, longest, 7)
     _check(checkers, _symmetric(rows, n), np.float32, ("block_pcg",))
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("n", [300, 6000])
+@pytest.mark.parametrize("longest", [127, 129, 299])
+def test_one_long_row(checkers, dtype, n, longest):
+    """Short rows and one of up to or more than 128 nonzeros: rows in registers, or staged tiles."""
+    lengths = np.full(n, 3)
+    lengths[n // 2] = 2 * (longest - 2) + 1  # its diagonal, its reach and the neighbour before it
+    matrix = _symmetric(lengths, longest)
+    assert np.diff(matrix[0]).max() == longest
+    _check(checkers, matrix, dtype, ("pcg", "cg", "block_pcg"))
