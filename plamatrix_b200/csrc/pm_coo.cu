@@ -102,14 +102,23 @@ __global__ void __launch_bounds__(256) count_kernel(const int64_t* __restrict__ 
 // kScatterWindow bytes, which stays in L2: pass 0 turns every slot into the record's position, the
 // others read that and, for their own triplets, the column and value again.  16M triplets of FP64:
 // 603 us in one pass, 456 in four (conversion 1,152 against 1,005 us; 128 MB windows 1,132, 48 MB 1,048).
+// Triplets that come in some order gain nothing from it: a warp whose records lie within one window's length
+// writes all of them in pass 0 and skips the others.  Conversions of 8-entry rows, us, in one pass /
+// this / windows for every warp, FP64: 16M shuffled 1,261 / 1,187 / 1,179; in row order 732 / 763 / 838;
+// rows within 10,000 of their place 879 / 893 / 1,010; FP32: 1,349 / 1,235 / 1,228, 765 / 802 / 862,
+// 1,005 / 1,028 / 1,123.
 constexpr size_t kScatterWindow = size_t(64) << 20;
-constexpr int kScatterPasses = 8; // a longer input re-reads more than it saves: one pass
+// Longer inputs take one pass: from six on the passes over ordered triplets cost what they save elsewhere
+// (25M of FP32: shuffled 2,135 in one pass, 1,943 in six; rows within 60,000 of their place 1,485 and 1,569).
+constexpr int kScatterPasses = 5;
+// a CTA's kPer * 256 triplets; ranges: every warp's least and greatest positions where pass 0 left some to the
+// others
 template <typename T, bool FIRST, int kPer>
-__global__ void __launch_bounds__(256) scatter_kernel(const int64_t* __restrict__ rows, const int64_t* __restrict__ cols,
-                                                      const T* __restrict__ values, int64_t count, int64_t col_count,
-                                                      int* __restrict__ slots, const int* __restrict__ bucket_start,
-                                                      CooRec<T>* __restrict__ recs, int64_t lo, int64_t hi,
-                                                      CooStatus* status)
+__device__ __forceinline__ void scatter_group(const int64_t* __restrict__ rows,
+                                              const int64_t* __restrict__ cols, const T* __restrict__ values,
+                                              int64_t count, int64_t col_count, int* __restrict__ slots,
+                                              const int* __restrict__ bucket_start, CooRec<T>* __restrict__ recs,
+                                              int64_t lo, int64_t hi, int2* __restrict__ ranges, CooStatus* status)
 {
     const int64_t i0 = int64_t(blockIdx.x) * (kPer * 256) + threadIdx.x;
     int pos[kPer];
@@ -127,10 +136,28 @@ __global__ void __launch_bounds__(256) scatter_kernel(const int64_t* __restrict_
                 pos[k] += bucket_start[__ldcs(rows + i0 + k * 256)];
         if (hi < count)
         {
+            int least = INT_MAX, greatest = -1;
 #pragma unroll
             for (int k = 0; k < kPer; ++k)
                 if (pos[k] >= 0)
-                    __stcs(slots + i0 + k * 256, pos[k]);
+                {
+                    least = min(least, pos[k]);
+                    greatest = max(greatest, pos[k]);
+                }
+            least = __reduce_min_sync(0xffffffffu, least);
+            greatest = __reduce_max_sync(0xffffffffu, greatest);
+            const bool left = greatest - least >= hi; // hi: a window's records
+            if (left)
+            {
+#pragma unroll
+                for (int k = 0; k < kPer; ++k)
+                    if (pos[k] >= 0)
+                        __stcs(slots + i0 + k * 256, pos[k]);
+            }
+            else
+                hi = count; // all of them here
+            if ((threadIdx.x & 31) == 0)
+                ranges[blockIdx.x * 8 + (threadIdx.x >> 5)] = left ? make_int2(least, greatest) : make_int2(INT_MAX, -1);
         }
     }
     int64_t col[kPer];
@@ -166,6 +193,29 @@ __global__ void __launch_bounds__(256) scatter_kernel(const int64_t* __restrict_
             recs[pos[k]] = r;
         }
     }
+}
+
+template <typename T, int kPer>
+__global__ void __launch_bounds__(256) scatter_kernel(const int64_t* __restrict__ rows, const int64_t* __restrict__ cols,
+                                                      const T* __restrict__ values, int64_t count, int64_t col_count,
+                                                      int* __restrict__ slots, const int* __restrict__ bucket_start,
+                                                      CooRec<T>* __restrict__ recs, int64_t hi,
+                                                      int2* __restrict__ ranges, CooStatus* status)
+{
+    scatter_group<T, true, kPer>(rows, cols, values, count, col_count, slots, bucket_start, recs, 0, hi,
+                                 ranges, status);
+}
+
+template <typename T, int kPer>
+__global__ void __launch_bounds__(256) scatter_window_kernel(const int64_t* __restrict__ cols,
+                                                             const T* __restrict__ values, int64_t count,
+                                                             int* __restrict__ slots, CooRec<T>* __restrict__ recs,
+                                                             int64_t lo, int64_t hi, int2* __restrict__ ranges)
+{
+    const int2 range = ranges[blockIdx.x * 8 + (threadIdx.x >> 5)];
+    if (range.y < lo || range.x >= hi)
+        return;
+    scatter_group<T, false, kPer>(nullptr, cols, values, count, 0, slots, nullptr, recs, lo, hi, nullptr, nullptr);
 }
 
 // odd-even merge network over N register-resident (key, value) pairs (63 comparators for 16; a
@@ -840,21 +890,21 @@ void coo_prepare(pm_sparse_workspace* ws, cudaStream_t stream, int64_t rows, int
         const bool windows = count > window && count <= kScatterPasses * window;
         // four triplets per thread once they fill the chip (2,048 threads per SM)
         const bool many = count > int64_t(sm_count()) * 2048 * 4;
-        const unsigned grid = grid_for(count, 4 * 256);
+        const unsigned groups = grid_for(count, 4 * 256);
+        int2* const ranges = reinterpret_cast<int2*>(ws->keys); // written by the sorts, after the passes
         if (many)
-            scatter_kernel<T, true, 4><<<grid, 256, 0, stream>>>(row_indices, col_indices, values, count, cols,
-                                                                 ws->slots, ws->bucket_start, recs, 0,
-                                                                 windows ? window : count, ws->status);
+            scatter_kernel<T, 4><<<groups, 256, 0, stream>>>(row_indices, col_indices, values, count, cols, ws->slots,
+                                                             ws->bucket_start, recs, windows ? window : count, ranges,
+                                                             ws->status);
         else
-            scatter_kernel<T, true, 1><<<grid_for(count, 256), 256, 0, stream>>>(
-                row_indices, col_indices, values, count, cols, ws->slots, ws->bucket_start, recs, 0, count,
-                ws->status);
+            scatter_kernel<T, 1><<<grid_for(count, 256), 256, 0, stream>>>(row_indices, col_indices, values, count,
+                                                                           cols, ws->slots, ws->bucket_start, recs,
+                                                                           count, ranges, ws->status);
         PM_LAUNCH_CHECK();
         for (int64_t lo = window; windows && lo < count; lo += window)
         {
-            scatter_kernel<T, false, 4><<<grid, 256, 0, stream>>>(row_indices, col_indices, values, count, cols,
-                                                                  ws->slots, ws->bucket_start, recs, lo, lo + window,
-                                                                  ws->status);
+            scatter_window_kernel<T, 4><<<groups, 256, 0, stream>>>(col_indices, values, count, ws->slots, recs, lo,
+                                                                    lo + window, ranges);
             PM_LAUNCH_CHECK();
         }
     }
