@@ -1665,11 +1665,11 @@ __device__ __forceinline__ bool schur_status_bad(const SchurStatus* s, int64_t o
            (s->observation_bad >= 0 && s->observation_bad < observations);
 }
 
-template <typename V, typename M, typename PM>
-__global__ void __launch_bounds__(32 * kLoopRows, 1) schur_pcg_kernel(const SchurLoop<V, M, PM> a)
+template <typename V, typename M, typename PM, int ROWS>
+__global__ void __launch_bounds__(32 * ROWS, 1) schur_pcg_kernel(const SchurLoop<V, M, PM> a)
 {
     __shared__ GridShared shared;
-    __shared__ PM blocks[kLoopRows][36];
+    __shared__ PM blocks[ROWS][36];
     if (a.status && schur_status_bad(a.status, a.observations))
         return; // nothing is solved; the host reports why
     SolveState* const st = a.st;
@@ -3153,15 +3153,27 @@ void queue_one_launch_pcg(pm_schur_workspace* ws, cudaStream_t stream, const M* 
     SchurLoop<V, M, PM> a{ws->P, ws->block_row_ptr, ws->block_col, S, minv, rhs, x, scratch, rel, abs_tol, rule,
                           max_iterations, window, x_is_zero, check, status, observations, ws->mail.packets(),
                           ws->mail.epoch, ws->state};
-    // one CTA while it holds all rows (its barriers are the cheapest), else the fewest rows per CTA
+    // One CTA while it holds all rows (its barriers are the cheapest), else at least eight rows each.  Rows
+    // longer than a warp's one round of loads are spread over all SMs; shorter ones take fewer CTAs, in steps
+    // of eight, because the barriers cost more than the loads (1,500 rows of 18 blocks, mixed precision: 309 us
+    // in 94 CTAs, 334 in 137; 1,500 rows of 282, FP64: 338 and 307), and so do more than 24 rows a CTA, which
+    // leave a row's loads 64 registers either way.
+    const int most = std::min(sm_count(), kGridMaxCtas);
     int rows = kLoopRows;
     if (ws->P > kLoopRows)
-        for (rows = 8; rows < kLoopRows && ws->P > int64_t(rows) * std::min(sm_count(), kGridMaxCtas);)
-            rows *= 2;
+    {
+        rows = std::max(8, static_cast<int>((ws->P + most - 1) / most));
+        if (ws->B <= 32 * ws->P || rows > 24)
+            rows = (rows + 7) / 8 * 8;
+    }
     PM_CUDA(cudaMemsetAsync(ws->state, 0, sizeof(SolveState), stream));
+    const auto kernel = rows <= 8    ? schur_pcg_kernel<V, M, PM, 8>
+                        : rows <= 16 ? schur_pcg_kernel<V, M, PM, 16>
+                        : rows <= 24 ? schur_pcg_kernel<V, M, PM, 24>
+                                     : schur_pcg_kernel<V, M, PM, 32>;
     void* args[] = {&a};
-    PM_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(schur_pcg_kernel<V, M, PM>),
-                                        dim3(grid_for(ws->P, rows)), dim3(32 * rows), args, 0, stream));
+    PM_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), dim3(grid_for(ws->P, rows)),
+                                        dim3(32 * rows), args, 0, stream));
     PM_LAUNCH_CHECK();
 }
 

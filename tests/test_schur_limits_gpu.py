@@ -3,8 +3,9 @@ import numpy as np
 import pytest
 import torch
 
-from gpu_util import host
+from gpu_util import dev, host
 from plamatrix_b200 import schur as SC
+from plamatrix_b200 import workloads as W
 
 pytestmark = pytest.mark.gpu
 
@@ -34,3 +35,24 @@ def test_no_primary_blocks(L, dtype):
     tolerance = 1e-12 if dtype == np.float64 else 1e-4
     error = np.linalg.norm(host(dl).reshape(-1, 3) - want, axis=1)
     assert np.all(error <= tolerance * np.linalg.norm(want, axis=1))
+
+
+@pytest.mark.parametrize("P", [9 * 148, 16 * 148, 17 * 148 + 3, 24 * 148, 24 * 148 + 1])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_block_rows_per_cta(checkers, P, dtype):
+    """Rows of more than 32 blocks, 9 to 25 of them in each CTA of the one-launch PCG.  Tolerances of the other
+    solve tests: 1e-6 (FP64) and 1e-4 (FP32) relative against the oracle, which solves to 1e-10."""
+    prob = W.bundle_problem(P, 20 * P, per_eliminated=4, window=24, seed=P)
+    ne = SC.DeviceNormalEquations(P, prob["L"], 6, 3, dtype)
+    ne.accumulate_observations(dev(prob["obs_primary"]), dev(prob["obs_eliminated"]), dev(prob["jp"].astype(dtype)),
+                               dev(prob["jl"].astype(dtype)), dev(prob["residual"].astype(dtype)), prob["huber_delta"])
+    want_p, want_l, _ = checkers.normal_equations_from_observations(prob).solve(
+        1e-3, relative_tolerance=1e-10, max_iterations=300)
+    ws = SC.SchurComplementSolverWorkspace()
+    tolerance = 1e-6 if dtype == np.float64 else 1e-4
+    options = SC.SchurComplementSolverOptions(max_iterations=300,
+                                              relative_tolerance=1e-10 if dtype == np.float64 else 1e-6)
+    dp, dl, rep = SC.solve_damped_schur_complement(ne, 1e-3, options, ws)
+    assert rep["converged"] and ws.dims()[2] > 32 * P
+    assert np.linalg.norm(host(dp) - want_p) <= tolerance * np.linalg.norm(want_p)
+    assert np.linalg.norm(host(dl) - want_l) <= tolerance * np.linalg.norm(want_l)
