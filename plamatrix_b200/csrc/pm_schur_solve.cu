@@ -2561,11 +2561,12 @@ constexpr int kUpperShapeCount = sizeof(kUpperShapes) / sizeof(kUpperShapes[0]);
 //   many pairs want all eight: 217.8 pairs, 156,000 blocks, FP64 2642 2671 2716 2660; 174 pairs, 11,700
 //     blocks, FP64 243 277 246 227;
 //   four lanes a pair keep 24 instead of 16 warps per SM, which pays with FP32 rows (217.8 pairs, FP32
-//     1935 1972 1851 1859) and with fewer blocks (27 pairs, 19,900 blocks, FP64 113 113 103 113);
+//     1935 1972 1851 1859) and with fewer blocks (27 pairs, 19,900 blocks, FP64 113 113 103 113; 93 pairs,
+//     45,150 blocks, FP64 335 329 349 355; 93 pairs, 11,700 blocks, FP64 348 412 367 333);
 //   below some 4,000 blocks a block's own chain is all there is: 63 pairs, 190 blocks, FP64 37 43 44 37.
 int default_shape(const pm_schur_workspace* ws, bool fp64)
 {
-    const bool split2 = fp64 && ws->U >= 65536;
+    const bool split2 = fp64 && ws->U >= 32768;
     if (ws->E < 64 * ws->U && ws->U >= 4096)
         return split2 ? 1 : 3;
     return split2 ? 0 : 4;
