@@ -17,6 +17,7 @@
 #include "pm_grid.cuh"
 #include "pm_piece.h"
 
+#include <atomic>
 #include <cmath>
 #include <limits>
 #include <sstream>
@@ -30,6 +31,7 @@ struct pm_csr
     const void* values = nullptr;
     int threads_per_row = 1; // lanes per row of the heuristic
     int longest_row = 0;     // its nonzeros
+    uint64_t serial = 0;     // no other operand of the process has it, also none that is created later
     int kernel = -1;         // -1: heuristic; 0: row-group stream; 1..32: lanes per row (autotuned or set)
 };
 
@@ -1375,7 +1377,8 @@ struct pm_solver_workspace
     // CG / PCG iteration graphs ('while' node around a chunk of iterations), one per operand set
     struct IterationGraph
     {
-        const void* key[5] = {};
+        uint64_t operand = 0; // its serial: an address may be another operand's by now
+        const void* key[4] = {};
         int64_t n = -1;
         int shape = 0, mode = -1, value_size = 0;
         int64_t block_size = 0;
@@ -1415,6 +1418,8 @@ namespace pm
 namespace
 {
 
+std::atomic<uint64_t> operand_count{0};
+
 template <typename T>
 void csr_create(cudaStream_t stream, int64_t rows, int64_t cols, int64_t nnz, const int64_t* ro, const int64_t* ci,
                 const T* v, pm_csr** out)
@@ -1436,6 +1441,7 @@ void csr_create(cudaStream_t stream, int64_t rows, int64_t cols, int64_t nnz, co
         A->nnz = nnz;
         A->values = v;
         A->threads_per_row = pick_tpr(rows, nnz);
+        A->serial = ++operand_count;
         PM_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&A->row_ptr), (rows + 1) * sizeof(int), stream));
         PM_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&A->col_idx), (nnz > 0 ? nnz : 1) * sizeof(int), stream));
         CsrCheck* check = nullptr;
@@ -1749,10 +1755,10 @@ cudaGraphExec_t cg_iteration_graph(pm_solver_workspace* ws, const pm_csr* A, T* 
 {
     const int64_t n = A->rows;
     const int shape = use_stream(A) ? 0 : lanes_per_row(A);
-    const void* key[5] = {A, A->values, x, blocks, ws->buffer.ptr};
+    const void* key[4] = {A->values, x, blocks, ws->buffer.ptr};
     for (auto& g : ws->graphs)
-        if (g.exec && g.n == n && g.shape == shape && g.mode == mode && g.block_size == bs &&
-            g.value_size == int(sizeof(T)) && std::equal(key, key + 5, g.key))
+        if (g.exec && g.operand == A->serial && g.n == n && g.shape == shape && g.mode == mode &&
+            g.block_size == bs && g.value_size == int(sizeof(T)) && std::equal(key, key + 4, g.key))
             return g.exec;
     if (!ws->capture_stream)
         PM_CUDA(cudaStreamCreateWithFlags(&ws->capture_stream, cudaStreamNonBlocking));
@@ -1812,7 +1818,8 @@ cudaGraphExec_t cg_iteration_graph(pm_solver_workspace* ws, const pm_csr* A, T* 
         cudaGraphDestroy(graph);
         fail(PM_CUDA_ERROR, std::string("CUDA iterative solver: iteration graph: ") + cudaGetErrorString(inst));
     }
-    std::copy(key, key + 5, slot.key);
+    slot.operand = A->serial;
+    std::copy(key, key + 4, slot.key);
     slot.n = n;
     slot.shape = shape;
     slot.mode = mode;

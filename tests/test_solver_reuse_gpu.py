@@ -1,0 +1,56 @@
+"""One solver workspace over operands that come and go, from several threads, and under a replayed capture."""
+import threading
+
+import numpy as np
+import pytest
+import torch
+
+from gpu_util import dev, host
+from plamatrix_b200 import sparse as S
+
+pytestmark = pytest.mark.gpu
+
+ROW1 = 512 * 148  # rows a chip of 148 SMs takes one to a thread
+
+
+def _banded(n, reach, seed):
+    """A symmetric band of `reach` on each side, its diagonal twice the absolute sum of the rest: condition
+    number below 30."""
+    rng = np.random.default_rng(seed)
+    i = np.concatenate([np.arange(n - d) for d in range(1, reach + 1)])
+    j = np.concatenate([np.arange(d, n) for d in range(1, reach + 1)])
+    v = rng.uniform(-1.0, 1.0, len(i))
+    weight = np.bincount(i, np.abs(v), n) + np.bincount(j, np.abs(v), n)
+    r, c = np.concatenate([np.arange(n), i, j]), np.concatenate([np.arange(n), j, i])
+    v = np.concatenate([2.0 * weight + 1.0, v, v])
+    order = np.lexsort((c, r))
+    offsets = np.zeros(n + 1, np.int64)
+    np.cumsum(np.bincount(r, minlength=n), out=offsets[1:])
+    return offsets, c[order], v[order]
+
+
+def test_operands_in_the_same_place(checkers):
+    """An operand is dropped and another is made over the same values, solution and block buffers, with more
+    and with fewer nonzeros: its solve is its own (FP32, blocks of six, more rows than one launch holds)."""
+    n = 96_000
+    rng = np.random.default_rng(1)
+    matrices = [_banded(n, reach, reach) for reach in (1, 3, 2)]
+    buffer = torch.empty(max(len(m[1]) for m in matrices), dtype=torch.float32, device="cuda")
+    solution = torch.empty(n, dtype=torch.float32, device="cuda")
+    inverse = torch.empty(6 * n, dtype=torch.float32, device="cuda")
+    b = rng.uniform(-1.0, 1.0, n).astype(np.float32)
+    ws = S.IterativeSolverWorkspace()
+    options = S.IterativeSolverOptions(relative_tolerance=1e-6)
+    for _ in range(3):
+        for ro, ci, v in matrices:
+            v = v.astype(np.float32)
+            buffer[:len(v)] = dev(v)
+            diagonal = v[np.repeat(np.arange(n), np.diff(ro)) == ci]
+            inverse.copy_(dev((np.eye(6)[None] / diagonal.reshape(-1, 6, 1)).reshape(-1).astype(np.float32)))
+            op = S.CsrOperand(S.CSRMatrix(n, n, dev(ro), dev(ci), buffer[:len(v)]))
+            solution.zero_()
+            report = S.block_pcg(op, dev(b), solution, inverse, 6, ws, options)
+            assert report["converged"]
+            want, _ = checkers.pcg(ro, ci, v.astype(np.float64), b.astype(np.float64), relative_tolerance=1e-12)
+            assert np.linalg.norm(host(solution) - want) <= 1e-4 * np.linalg.norm(want)
+            del op
