@@ -160,11 +160,12 @@ struct GridMail
     }
 };
 
-// more than the default 48 KB of shared memory, static arrays included
-inline void allow_smem(const void* kernel, size_t bytes)
+// More than the default 48 KB of shared memory, static arrays included.  The limit is the function's, not the
+// launch's: `most` is the same in every call for a kernel, so that no thread lowers another's.
+inline void allow_smem(const void* kernel, size_t most)
 {
-    if (bytes > 40 * 1024)
-        PM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)));
+    if (most > 40 * 1024)
+        PM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(most)));
 }
 
 } // namespace pm

@@ -54,3 +54,39 @@ def test_operands_in_the_same_place(checkers):
             want, _ = checkers.pcg(ro, ci, v.astype(np.float64), b.astype(np.float64), relative_tolerance=1e-12)
             assert np.linalg.norm(host(solution) - want) <= 1e-4 * np.linalg.norm(want)
             del op
+
+
+@pytest.mark.parametrize("sizes", [(4 * ROW1 + 777, 8 * ROW1), (3000, ROW1 - 5), (2 * ROW1 + 40, 4 * ROW1 - 3)])
+def test_two_sizes_of_one_kernel_at_once(sizes):
+    """Two threads solve systems that take the same kernel with different shared memory, each with its own
+    workspace and stream: every solve runs and gives the bits of one alone."""
+    ops, rhs, want = [], [], []
+    for n in sizes:
+        ro, ci, v = _banded(n, 2, n)
+        ops.append(S.CsrOperand(S.CSRMatrix(n, n, dev(ro), dev(ci), dev(v))))
+        rhs.append(torch.linspace(-1.0, 1.0, n, dtype=torch.float64, device="cuda"))
+        want.append(torch.zeros_like(rhs[-1]))
+        S.pcg(ops[-1], rhs[-1], want[-1])
+    torch.cuda.synchronize()
+    got, failures = [[], []], []
+
+    def solve(k):
+        try:
+            stream, ws = torch.cuda.Stream(), S.IterativeSolverWorkspace()
+            with torch.cuda.stream(stream):
+                for _ in range(40):
+                    x = torch.zeros_like(rhs[k])
+                    S.pcg(ops[k], rhs[k], x, ws, stream=stream)
+                    got[k].append(x)
+            stream.synchronize()
+            ws.close()
+        except Exception as error:  # a thread's exception would be lost
+            failures.append(error)
+
+    threads = [threading.Thread(target=solve, args=(k,)) for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failures
+    assert all(len(got[k]) == 40 and all(torch.equal(x, want[k]) for x in got[k]) for k in range(2))
