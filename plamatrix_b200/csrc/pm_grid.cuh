@@ -46,7 +46,7 @@ struct GridShared // of one CTA
 
 struct GridSync
 {
-    Packet* mail; // [2][CTA][CTA][2], epochs below this solve's before the launch
+    Packet* mail; // [2][CTA][CTA][2], epochs below this launch's before it
     int* timed_out; // device flag: a barrier gave up
     GridShared* sh;
     unsigned long long epoch;
@@ -141,22 +141,30 @@ __device__ __forceinline__ bool grid_barrier(GridSync& g)
     return grid_sum<1>(g, none, total, true);
 }
 
-// the mailboxes of one workspace, zeroed once; every launch takes barrier numbers of its own
+// The mailboxes of one workspace and the number below which all its barriers lie so far, zeroed once.  Every
+// launch takes numbers of its own from the device, through grid_next_launch in a kernel queued before it: a
+// captured launch is replayed with the same arguments, and packets of the replay before must not pass for its own.
+constexpr size_t kGridPackets = 4 * size_t(kGridMaxCtas) * kGridMaxCtas;
+
+__device__ __forceinline__ void grid_next_launch(unsigned long long* epoch)
+{
+    *epoch += 1ull << 34; // more than the barriers of any solve (three per iteration)
+}
+
 struct GridMail
 {
     DeviceBuffer buffer;
-    unsigned long long epoch = 0;
     Packet* packets() const { return static_cast<Packet*>(buffer.ptr); }
+    unsigned long long* epoch() const { return reinterpret_cast<unsigned long long*>(packets() + kGridPackets); }
     void open(cudaStream_t stream, const char* owner)
     {
         buffer.bind(stream, owner);
         if (!buffer.ptr)
         {
-            const size_t bytes = 4 * size_t(kGridMaxCtas) * kGridMaxCtas * sizeof(Packet);
+            const size_t bytes = (kGridPackets + 1) * sizeof(Packet);
             buffer.ensure(bytes, stream, owner);
             PM_CUDA(cudaMemsetAsync(buffer.ptr, 0, bytes, stream));
         }
-        epoch += 1ull << 34; // more than the barriers of any solve (three per iteration)
     }
 };
 

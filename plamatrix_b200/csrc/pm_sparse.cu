@@ -553,7 +553,7 @@ struct PcgLoop
     int64_t bs;
     double relative, absolute;
     Packet* mail;             // [2][CTA][CTA][2]
-    unsigned long long epoch; // barriers of earlier solves end below it
+    const unsigned long long* epoch; // barriers of earlier launches end below it
     PcgState* st;
 };
 
@@ -738,7 +738,7 @@ __global__ void __launch_bounds__(loop_threads<T>(SHAPE), 1) pcg_loop_kernel(con
     __shared__ GridShared shared;
     PcgState* const st = a.st;
     constexpr bool FUSE = !KEEP;
-    GridSync sync{a.mail, &st->timed_out, &shared, a.epoch};
+    GridSync sync{a.mail, &st->timed_out, &shared, *a.epoch};
     if (threadIdx.x == 0)
         shared.failed = 0; // read after the first barrier's __syncthreads
     // a row's lane owns its entries in the vector phases too (block rows read their neighbours' q)
@@ -923,7 +923,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) pcg_row_kernel(const PcgLoop<T
     extern __shared__ __align__(16) unsigned char loop_smem[];
     __shared__ GridShared shared;
     PcgState* const st = a.st;
-    GridSync sync{a.mail, &st->timed_out, &shared, a.epoch};
+    GridSync sync{a.mail, &st->timed_out, &shared, *a.epoch};
     if (threadIdx.x == 0)
         shared.failed = 0; // read after the first barrier's __syncthreads
     const int lane = threadIdx.x & 31;
@@ -1333,8 +1333,9 @@ __global__ void cg_continue_kernel(cudaGraphConditionalHandle handle, PcgState* 
     }
 }
 
-__global__ void pcg_reset_kernel(PcgState* st, int max_iterations)
+__global__ void pcg_reset_kernel(PcgState* st, int max_iterations, unsigned long long* epoch)
 {
+    grid_next_launch(epoch);
     PcgState s{};
     s.max_iterations = max_iterations;
     s.jacobi_bad_row = kNone;
@@ -1932,10 +1933,10 @@ PcgState* queue_pcg(pm_solver_workspace* ws, const pm_csr* A, const T* b, T* x, 
     const PcgVectors<T> u(ws, n);
     ws->mail.open(stream, "IterativeSolverWorkspace");
     const T* v = static_cast<const T*>(A->values);
-    pcg_reset_kernel<<<1, 1, 0, stream>>>(u.st, max_iterations);
+    pcg_reset_kernel<<<1, 1, 0, stream>>>(u.st, max_iterations, ws->mail.epoch());
     PM_LAUNCH_CHECK();
     PcgLoop<T> a{n, static_cast<int>(A->nnz), A->row_ptr, A->col_idx, v, b, x, {u.r[0], u.r[1]}, u.z, {u.p[0], u.p[1]},
-                 u.q, u.inv, mode, blocks, bs, relative, absolute, ws->mail.packets(), ws->mail.epoch, u.st};
+                 u.q, u.inv, mode, blocks, bs, relative, absolute, ws->mail.packets(), ws->mail.epoch(), u.st};
     if (launch_pcg_loop<T>(A, a, stream))
         return u.st;
     if (mode == 1)
@@ -2165,6 +2166,7 @@ void pm_fixed_state_destroy(pm_fixed_state* state)
         if (state->event)
             cudaEventSynchronize(state->event);
         delete state;
+        cudaGetLastError(); // a captured event cannot be waited for: not the next call's error
     }
 }
 

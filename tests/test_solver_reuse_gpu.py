@@ -90,3 +90,53 @@ def test_two_sizes_of_one_kernel_at_once(sizes):
         t.join()
     assert not failures
     assert all(len(got[k]) == 40 and all(torch.equal(x, want[k]) for x in got[k]) for k in range(2))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("n", [3000, 2 * ROW1, 5 * ROW1])
+def test_replayed_capture(dtype, n):
+    """A fixed-iteration solve captured once: every replay gives the bits of a direct call, also between
+    direct calls with the same workspace."""
+    ro, ci, v = _banded(n, 2, n)
+    op = S.CsrOperand(S.CSRMatrix(n, n, dev(ro), dev(ci), dev(v, dtype)))
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n)
+    sides = [torch.rand(n, generator=g, device="cuda", dtype=torch.float64).to(dtype) - 0.5 for _ in range(6)]
+    b, x = torch.empty_like(sides[0]), torch.empty_like(sides[0])
+    stream, ws = torch.cuda.Stream(), S.IterativeSolverWorkspace()
+    held = []
+
+    def solve(target):
+        target.zero_()
+        held.append(S.pcg_fixed_iterations_async(op, b, target, 25, ws, stream=stream))
+
+    torch.cuda.synchronize()
+    want = []
+    with torch.cuda.stream(stream):
+        for side in sides:  # one after the other: also the workspace's first growth
+            b.copy_(side)
+            y = torch.empty_like(b)
+            solve(y)
+            stream.synchronize()
+            want.append(y)
+        assert not torch.equal(want[0], want[1])
+        graph = torch.cuda.CUDAGraph()
+        graph.capture_begin(capture_error_mode="relaxed")
+        solve(x)
+        graph.capture_end()
+        for _ in range(3):
+            for k, side in enumerate(sides):
+                b.copy_(side)
+                graph.replay()
+                if k % 3 == 1:
+                    y = torch.empty_like(b)
+                    solve(y)
+                    stream.synchronize()
+                    assert torch.equal(y, want[k])
+                stream.synchronize()
+                assert torch.equal(x, want[k])
+    stream.synchronize()
+    del graph
+    held.clear()
+    # nothing of the captured event is left over for the next call
+    S.pcg(op, sides[0], torch.zeros_like(x))
