@@ -405,7 +405,8 @@ PM_API int pm_schur_solve_f64(pm_schur_workspace* workspace, pm_stream_t stream,
  * pm_schur_assembly_shape_count() lane layouts ({pair streams, lanes per pair}); each sums every
  * block in a fixed order of its own, so a shape gives repeatable values, and shapes differ from
  * one another only by rounding.  A workspace whose caller sets none takes the shape from the system's
- * pairs per block, block count and type.  pm_schur_autotune_assembly times every shape `repeats` times on
+ * pairs per block, block count and type; pm_schur_assembly_shape then reports that of the last assembly
+ * (0 before the first), and setting it in another workspace gives the same bits.  pm_schur_autotune_assembly times every shape `repeats` times on
  * the system `workspace` last solved (`equations` must be that system), keeps the fastest in the
  * workspace and reports its index, its mean ms and (shape_ms_h, may be NULL, one per shape)
  * every shape's mean ms.  It reassembles the system, so the workspace needs a new solve before

@@ -104,7 +104,8 @@ struct pm_schur_workspace
     int2* pairs = nullptr;         // E: {row-list entry of cross (l, p), row-list entry of cross (l, q)}, per block in ascending l
     void* vfactor = nullptr;       // C x 18 (Scalar): V = W_lp L_l^-T of every row-list entry (written by the diagonal pass)
     bool shape_pinned = false;     // the caller or the autotuner chose upper_shape
-    int upper_shape = 0;           // launch shape of the upper-block pass (index into kUpperShapes)
+    int upper_shape = 0;           // launch shape of the upper-block pass (index into kUpperShapes): the chosen
+                                   // one, or that of the last assembly
     int* saved_offsets = nullptr;
     int* saved_primary = nullptr;
     int* saved_pc = nullptr;
@@ -2551,8 +2552,8 @@ void build_pattern(pm_schur_workspace* ws, const pm_normal_equations* ne, cudaSt
     ws->pattern_builds += 1;
 }
 
-// Launch shapes of the upper-block pass: {pair streams, lanes per pair}.  Shape 0 is the default;
-// pm_schur_autotune_assembly times them all on the caller's system and keeps the fastest.
+// Launch shapes of the upper-block pass: {pair streams, lanes per pair}.  default_shape picks one of four by
+// rule; pm_schur_autotune_assembly times them all on the caller's system and keeps the fastest.
 struct UpperShape
 {
     int streams, split;
@@ -2592,7 +2593,9 @@ template <typename TO, typename TP, typename VT, typename AT>
 void launch_upper(pm_schur_workspace* ws, const int* block_pc, const VT* vf, const TP* pcv, TO* S,
                   cudaStream_t stream)
 {
-    switch (ws->shape_pinned ? ws->upper_shape : default_shape(ws, sizeof(VT) == 8))
+    if (!ws->shape_pinned)
+        ws->upper_shape = default_shape(ws, sizeof(VT) == 8);
+    switch (ws->upper_shape)
     {
     case 1: launch_upper_shape<TO, TP, VT, AT, 4, 2>(ws, block_pc, vf, pcv, S, stream); break;
     case 2: launch_upper_shape<TO, TP, VT, AT, 16, 2>(ws, block_pc, vf, pcv, S, stream); break;
@@ -4119,15 +4122,32 @@ void autotune_assembly(pm_schur_workspace* ws, cudaStream_t stream, const pm_nor
         return;
     }
     const bool fp32 = ws->s32_only;
-    cudaEvent_t e0 = nullptr, e1 = nullptr;
+    struct Tuning // a call that fails leaves the choice as it was
+    {
+        pm_schur_workspace* ws;
+        int shape = ws->upper_shape;
+        bool pinned = ws->shape_pinned;
+        cudaEvent_t e0 = nullptr, e1 = nullptr;
+        ~Tuning()
+        {
+            ws->upper_shape = shape;
+            ws->shape_pinned = pinned;
+            ws->assembled = false; // values and their FP32 copies now belong to the last shape timed
+            if (e0)
+                cudaEventDestroy(e0);
+            if (e1)
+                cudaEventDestroy(e1);
+        }
+    } tuning{ws};
+    cudaEvent_t &e0 = tuning.e0, &e1 = tuning.e1;
     PM_CUDA(cudaEventCreate(&e0));
     PM_CUDA(cudaEventCreate(&e1));
     double best = 0.0;
     int chosen = -1;
+    ws->shape_pinned = true;
     for (int k = 0; k < kUpperShapeCount; ++k)
     {
         ws->upper_shape = k;
-        ws->shape_pinned = true;
         launch_assembly<T>(ws, ne, ws->damping, ws->min_diag, stream, fp32); // warm-up
         PM_CUDA(cudaEventRecord(e0, stream));
         for (int r = 0; r < repeats; ++r)
@@ -4145,10 +4165,8 @@ void autotune_assembly(pm_schur_workspace* ws, cudaStream_t stream, const pm_nor
             chosen = k;
         }
     }
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    ws->upper_shape = chosen;
-    ws->assembled = false; // values and their FP32 copies now belong to the last shape timed
+    tuning.shape = chosen;
+    tuning.pinned = true;
     *shape = chosen;
     *best_ms = best;
 }

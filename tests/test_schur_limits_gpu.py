@@ -56,3 +56,23 @@ def test_block_rows_per_cta(checkers, P, dtype):
     assert rep["converged"] and ws.dims()[2] > 32 * P
     assert np.linalg.norm(host(dp) - want_p) <= tolerance * np.linalg.norm(want_p)
     assert np.linalg.norm(host(dl) - want_l) <= tolerance * np.linalg.norm(want_l)
+
+
+@pytest.mark.parametrize("P, L, k", [(30, 1500, 4), (120, 3000, 4), (120, 40000, 6), (420, 30000, 4), (420, 250000, 12)])
+@pytest.mark.parametrize("precision", ["native", "mixed_fp32_assembly"])
+def test_reported_shape_gives_the_bits(P, L, k, precision):
+    """Few and many blocks, few and many pairs in each: the shape that a workspace reports after a solve, set in
+    another one, assembles the same values."""
+    prob = W.bundle_problem_device(P, L, per_eliminated=k, seed=P)
+    ne = SC.DeviceNormalEquations(P, L, 6, 3)
+    ne.accumulate_observations(*(prob[key] for key in ("obs_primary", "obs_eliminated", "jp", "jl", "residual")), 1.0)
+    options = SC.SchurComplementSolverOptions(max_iterations=300, relative_tolerance=1e-8, precision=precision)
+    free, pinned = SC.SchurComplementSolverWorkspace(), SC.SchurComplementSolverWorkspace()
+    SC.solve_damped_schur_complement(ne, 1e-3, options, free)
+    pinned.assembly_shape = free.assembly_shape
+    SC.solve_damped_schur_complement(ne, 1e-3, options, pinned)
+    assert torch.equal(free.export()["values"], pinned.export()["values"])
+    # a shape that is chosen stays, whatever the rule says
+    pinned.assembly_shape = 6
+    SC.solve_damped_schur_complement(ne, 1e-3, options, pinned)
+    assert pinned.assembly_shape == 6
