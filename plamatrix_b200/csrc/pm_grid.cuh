@@ -176,4 +176,20 @@ inline void allow_smem(const void* kernel, size_t most)
         PM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(most)));
 }
 
+// A launch whose CTAs wait for one another; false where the device will not hold all of them at once (a
+// context with fewer SMs than the device has): the caller then takes its kernels one by one.
+inline bool launch_resident(const void* kernel, unsigned ctas, unsigned threads, void** args, size_t smem,
+                            cudaStream_t stream)
+{
+    const cudaError_t launched = cudaLaunchCooperativeKernel(kernel, dim3(ctas), dim3(threads), args, smem, stream);
+    if (launched == cudaErrorCooperativeLaunchTooLarge)
+    {
+        cudaGetLastError(); // not the next launch's error
+        return false;
+    }
+    check_cuda(launched, "cooperative launch");
+    PM_LAUNCH_CHECK();
+    return true;
+}
+
 } // namespace pm

@@ -3151,10 +3151,10 @@ inline bool one_launch_pcg(const pm_schur_workspace* ws)
     return ws->bp == 6 && ws->P > 0 && ws->P <= int64_t(kLoopRows) * std::min(sm_count(), kGridMaxCtas);
 }
 
-// Queues it.  check: the FP64 true residual of the step; status: solve only if the factorisations
-// succeeded and no observation was rejected
+// Queues it; false where the device will not hold it.  check: the FP64 true residual of the step; status: solve
+// only if the factorisations succeeded and no observation was rejected
 template <typename V, typename M, typename PM>
-void queue_one_launch_pcg(pm_schur_workspace* ws, cudaStream_t stream, const M* S, const PM* minv, const double* rhs,
+bool queue_one_launch_pcg(pm_schur_workspace* ws, cudaStream_t stream, const M* S, const PM* minv, const double* rhs,
                           V* x, double rel, double abs_tol, int rule, int max_iterations, V* scratch, int window,
                           bool x_is_zero, bool check = false, const SchurStatus* status = nullptr,
                           int64_t observations = 0)
@@ -3183,9 +3183,7 @@ void queue_one_launch_pcg(pm_schur_workspace* ws, cudaStream_t stream, const M* 
                         : rows <= 24 ? schur_pcg_kernel<V, M, PM, 24>
                                      : schur_pcg_kernel<V, M, PM, 32>;
     void* args[] = {&a};
-    PM_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), dim3(grid_for(ws->P, rows)),
-                                        dim3(32 * rows), args, 0, stream));
-    PM_LAUNCH_CHECK();
+    return launch_resident(reinterpret_cast<const void*>(kernel), grid_for(ws->P, rows), 32 * rows, args, 0, stream);
 }
 
 // the device state, read after everything queued so far
@@ -3207,12 +3205,10 @@ SolveState block_pcg(pm_schur_workspace* ws, cudaStream_t stream, const M* S, co
                      V* x, double rel, double abs_tol, int rule, int max_iterations, V* scratch, int window = 0,
                      bool x_is_zero = false)
 {
-    if (one_launch_pcg(ws))
-    {
+    if (one_launch_pcg(ws) &&
         queue_one_launch_pcg<V, M, PM>(ws, stream, S, minv, rhs, x, rel, abs_tol, rule, max_iterations, scratch,
-                                       window, x_is_zero);
+                                       window, x_is_zero))
         return read_solve_state(ws, stream);
-    }
     const int64_t P = ws->P, n = ws->P * ws->bp;
     const int bp = static_cast<int>(ws->bp);
     V* r0 = scratch;
@@ -3715,7 +3711,7 @@ void schur_solve(pm_schur_workspace* ws, cudaStream_t stream, const pm_normal_eq
     // ---- status of the factorisations (one small read; the reference returns early here).  A plain
     // solve in one launch queues everything first, on the condition of that status, and reads once.
     double* area = vector_area(ws);
-    const bool queued = !mixed && !dense && !batch && !o->learned && one_launch_pcg(ws);
+    bool queued = !mixed && !dense && !batch && !o->learned && one_launch_pcg(ws);
     PM_CUDA(cudaMemcpyAsync(ws->host_status, ws->status, sizeof(SchurStatus), cudaMemcpyDeviceToHost, stream));
     // dl from dp: always, or only if the device state says that the solve converged
     bool t_at_step = false;
@@ -3752,13 +3748,14 @@ void schur_solve(pm_schur_workspace* ws, cudaStream_t stream, const pm_normal_eq
         PM_LAUNCH_CHECK();
     };
     SolveState queued_state{};
+    queued = queued &&
+             queue_one_launch_pcg<T, T, double>(ws, stream, static_cast<const T*>(ws->S), ws->minv, ws->rhs, dp,
+                                                o->relative_tolerance, o->absolute_tolerance, o->tolerance_rule,
+                                                o->max_iterations, reinterpret_cast<T*>(area), 0,
+                                                !o->use_initial_guess, o->check_true_residual && sizeof(T) == 8,
+                                                ws->status, ne->observation_status.ptr ? ne->observation_count : 0);
     if (queued)
     {
-        queue_one_launch_pcg<T, T, double>(ws, stream, static_cast<const T*>(ws->S), ws->minv, ws->rhs, dp,
-                                           o->relative_tolerance, o->absolute_tolerance, o->tolerance_rule,
-                                           o->max_iterations, reinterpret_cast<T*>(area), 0, !o->use_initial_guess,
-                                           o->check_true_residual && sizeof(T) == 8, ws->status,
-                                           ne->observation_status.ptr ? ne->observation_count : 0);
         PM_CUDA(cudaEventRecord(ws->events[4], stream));
         back_substitute(ws->state);
         PM_CUDA(cudaEventRecord(ws->events[5], stream));

@@ -1833,14 +1833,12 @@ cudaGraphExec_t cg_iteration_graph(pm_solver_workspace* ws, const pm_csr* A, T* 
 
 // smem: this launch's shared memory, most_smem: that of the kernel's largest launch
 template <typename T, typename Kernel>
-void launch_cooperative(Kernel kernel, PcgLoop<T>& a, unsigned ctas, unsigned threads, size_t smem, size_t most_smem,
+bool launch_cooperative(Kernel kernel, PcgLoop<T>& a, unsigned ctas, unsigned threads, size_t smem, size_t most_smem,
                         cudaStream_t stream)
 {
     allow_smem(reinterpret_cast<const void*>(kernel), most_smem);
     void* args[] = {&a};
-    PM_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), dim3(ctas), dim3(threads), args, smem,
-                                        stream));
-    PM_LAUNCH_CHECK();
+    return launch_resident(reinterpret_cast<const void*>(kernel), ctas, threads, args, smem, stream);
 }
 
 // One cooperative launch of the whole solve where it is the faster form (see pcg_loop_kernel);
@@ -1867,9 +1865,8 @@ bool launch_pcg_loop_shape(PcgLoop<T>& a, size_t warp_smem, int lanes, int longe
                 if (a.n > int64_t(block) * per_thread * most)
                     block = kRowThreads;
                 const size_t warp = size_t(kTileCap) * per_thread * (sizeof(T) + sizeof(int));
-                launch_cooperative(kernel, a, grid_for(a.n, static_cast<int>(block) * per_thread, most), block,
-                                   warp * (block / 32), warp * (kRowThreads / 32), stream);
-                return true;
+                return launch_cooperative(kernel, a, grid_for(a.n, static_cast<int>(block) * per_thread, most), block,
+                                          warp * (block / 32), warp * (kRowThreads / 32), stream);
             };
             if (a.n <= int64_t(kRowThreads) * most)
                 return launch_rows(pcg_row_kernel<T, 1>, 1);
@@ -1882,11 +1879,7 @@ bool launch_pcg_loop_shape(PcgLoop<T>& a, size_t warp_smem, int lanes, int longe
         const size_t kept = size_t(per_thread) * kTileThreads * sizeof(T);
         const size_t staged = kTileThreads / 32 * 2 * sizeof(RowTile<T, kKeepCap>);
         if (a.mode != 2 && kept <= kSmem - staged)
-        {
-            launch_cooperative(pcg_loop_kernel<T, 1, true>, a, ctas, kTileThreads, staged + kept, kSmem,
-                               stream);
-            return true;
-        }
+            return launch_cooperative(pcg_loop_kernel<T, 1, true>, a, ctas, kTileThreads, staged + kept, kSmem, stream);
         warp_smem = 2 * sizeof(RowTile<T, kTileCap>);
     }
     if ((SHAPE == -1 || (SHAPE == 1 && sizeof(T) == 4)) && longest_row > kLoneRow)
@@ -1899,9 +1892,8 @@ bool launch_pcg_loop_shape(PcgLoop<T>& a, size_t warp_smem, int lanes, int longe
     unsigned threads = 256;
     while (threads < kMost && wanted > int64_t(threads) * most)
         threads = std::min(2 * threads, kMost);
-    launch_cooperative(pcg_loop_kernel<T, SHAPE, false>, a, grid_for(wanted, static_cast<int>(threads), most), threads,
-                       warp_smem * (threads / 32), warp_smem * (kMost / 32), stream);
-    return true;
+    return launch_cooperative(pcg_loop_kernel<T, SHAPE, false>, a, grid_for(wanted, static_cast<int>(threads), most),
+                              threads, warp_smem * (threads / 32), warp_smem * (kMost / 32), stream);
 }
 
 template <typename T>
