@@ -1698,8 +1698,11 @@ struct PcgVectors
         c.base = static_cast<char*>(ws->buffer.ptr);
         st = c.take<PcgState>(1);
         partials = c.take<double>(3 * kMaxReduceBlocks);
-        for (T** v : {&r[0], &r[1], &z, &p[0], &p[1], &q, &inv})
+        for (T** v : {&r[0], &r[1], &z, &p[0], &q, &inv})
             *v = c.take<T>(n);
+        // only the launches that form p inside the SpMV keep the old one beside it: one row per thread or group
+        // of lanes, or four with rows in registers
+        p[1] = n <= int64_t(4) * kRowThreads * kGridMaxCtas ? c.take<T>(n) : nullptr;
         bytes = c.offset;
     }
 };

@@ -140,3 +140,24 @@ def test_replayed_capture(dtype, n):
     held.clear()
     # nothing of the captured event is left over for the next call
     S.pcg(op, sides[0], torch.zeros_like(x))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+def test_workspace_of_a_large_solve(dtype):
+    """Six vectors and small arrays (partial sums and mailboxes, below 4 MB), with the residual kept on the chip
+    and as kernels."""
+    runtime = pytest.importorskip("cuda.bindings.runtime")
+    size = torch.finfo(dtype).bits // 8
+    for n in (400_000, 5_000_000):
+        offsets, diagonal = torch.arange(n + 1, device="cuda"), torch.arange(n, device="cuda")
+        op = S.CsrOperand(S.CSRMatrix(n, n, offsets, diagonal, torch.full((n,), 2.0, dtype=dtype, device="cuda")))
+        b, x = torch.ones(n, dtype=dtype, device="cuda"), torch.zeros(n, dtype=dtype, device="cuda")
+        torch.cuda.synchronize()
+        _, pool = runtime.cudaDeviceGetDefaultMemPool(0)
+        used = runtime.cudaMemPoolAttr.cudaMemPoolAttrUsedMemCurrent
+        before = int(runtime.cudaMemPoolGetAttribute(pool, used)[1])
+        ws = S.IterativeSolverWorkspace()
+        assert S.pcg(op, b, x, ws)["converged"]
+        after = int(runtime.cudaMemPoolGetAttribute(pool, used)[1])
+        assert 0 < after - before <= 6 * n * size + (4 << 20)
+        ws.close()
