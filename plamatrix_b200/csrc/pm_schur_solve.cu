@@ -4193,6 +4193,11 @@ int pm_schur_workspace_close(pm_schur_workspace* ws)
         ws->pattern.release();
         ws->numeric.release();
         ws->scratch.release();
+        ws->dense.release();
+        ws->pair_buffer.release();
+        ws->mail.buffer.release();
+        if (ws->prim_sort)
+            pm_sparse_workspace_close(ws->prim_sort);
         ws->pattern_builds = ws->pattern_builds; // the count survives, the cache does not
         ws->saved_offsets = nullptr;
         ws->status = nullptr;
