@@ -1013,7 +1013,9 @@ int coo_async(pm_sparse_workspace* ws, cudaStream_t stream, int64_t rows, int64_
             fail(PM_RUNTIME_ERROR, "cooToCsrAsync empty input requires output nnz=0");
         }
         require_values(count, v);
-        coo_prepare<T>(ws, stream, rows, cols, count, ri, ci, v, false, true);
+        // an output that the fill refuses leaves the count behind it, with its status
+        const bool fills = nnz >= 0 && ro && (nnz == 0 || (co && vo));
+        coo_prepare<T>(ws, stream, rows, cols, count, ri, ci, v, false, fills);
         coo_fill<T>(ws, stream, nnz, ro, co, vo, true);
     });
 }
