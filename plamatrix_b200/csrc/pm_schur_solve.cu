@@ -1868,8 +1868,6 @@ __device__ __forceinline__ void cross_run(CrossRun& run, int lo, int hi, int cb,
                                           const int* __restrict__ cross_primary, const double* __restrict__ w,
                                           const double* __restrict__ x, Product&& product, Fold&& fold)
 {
-    if (cb >= ce) // uniform in the warp: nothing is read (x may be empty: a problem of no primaries)
-        return;
     const int lane = threadIdx.x & 31;
     auto stage = [&](int c0, int buffer) { // crosses c0 .. c0 + 31, those before ce
         const int pieces = min(32, ce - c0) * 9;
@@ -1894,8 +1892,11 @@ __device__ __forceinline__ void cross_run(CrossRun& run, int lo, int hi, int cb,
     int primary = cb + lane < ce ? cross_primary[cb + lane] : 0;
     int primary_next = cb + 32 + lane < ce ? cross_primary[cb + 32 + lane] : 0;
     double xv[6], xn[6];
-    stage(cb, 0);
-    gather(primary, xv);
+    if (cb < ce) // uniform in the warp; x may be empty (a problem of no primaries)
+    {
+        stage(cb, 0);
+        gather(primary, xv);
+    }
     int buffer = 0;
     for (int c0 = cb; c0 < ce; c0 += 32, buffer ^= 1)
     {
