@@ -582,7 +582,8 @@ template <typename T>
 __device__ __forceinline__ void jacobi_row(int64_t r, const int* __restrict__ rp, const int* __restrict__ ci,
                                            const T* __restrict__ v, T* inv, PcgState* st)
 {
-    double diag = 0.0, scale = 0.0;
+    double diag = 0.0;
+    T most = T(0);
     bool found = false;
     constexpr int G = 8; // loads in flight
     const int* c = ci + rp[r];
@@ -602,7 +603,7 @@ __device__ __forceinline__ void jacobi_row(int64_t r, const int* __restrict__ rp
         for (int k = 0; k < G; ++k)
             if (k < left)
             {
-                scale = fmax(scale, fabs(static_cast<double>(value[k])));
+                most = max(most, abs(value[k]));
                 if (col[k] == r)
                 {
                     diag += static_cast<double>(value[k]);
@@ -610,7 +611,7 @@ __device__ __forceinline__ void jacobi_row(int64_t r, const int* __restrict__ rp
                 }
             }
     }
-    const double threshold = Eps<T>::value * scale * 16.0;
+    const double threshold = Eps<T>::value * static_cast<double>(most) * 16.0;
     const double reciprocal = 1.0 / diag;
     if (!found || !isfinite(diag) || diag <= threshold || !isfinite(reciprocal))
     {
