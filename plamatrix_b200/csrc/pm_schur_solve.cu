@@ -2,8 +2,8 @@
 // solveDampedSchurComplement (src/optimization/block_schur.cpp:54-459) with its reusable
 // Schur pattern (src/optimization/block_schur_sparse_assembly.h:41-260, 472-520).
 //
-// Pipeline (all on one stream, no host round trip except the pattern-cache check and the
-// convergence polls):
+// Pipeline (all on one stream; the host reads the pattern-cache check, the factorisations' status
+// and the solver's final state, in mixed precision once per refinement step):
 //   1. eliminated blocks: damping H_ii += lambda * max(|H_ii|, minDiag), FP64 Cholesky
 //      inverse, y_l = Hll^-1 g_l                                (one thread per block)
 //   2. pattern (only when the topology changed): per-primary cross lists, block-CSR rows
@@ -1672,6 +1672,9 @@ __global__ void solve_reset_kernel(SolveState* st, unsigned long long* epoch)
     grid_next_launch(epoch);
 }
 
+// ROWS: the most rows (warps) of a CTA, which gives a thread 214, 128, 80 or 64 registers with 8, 16, 24 or 32: the
+// loads of a row's blocks that can be in flight (FP64, 1,000 rows of 985 blocks, 8 rows a CTA: 1,155 us at 64,
+// 481 at 214, 716 as a graph; 3,000 rows of 555, 21 a CTA: 895 at 64, 760 at 80, 826 as a graph).
 template <typename V, typename M, typename PM, int ROWS>
 __global__ void __launch_bounds__(32 * ROWS, 1) schur_pcg_kernel(const SchurLoop<V, M, PM> a)
 {

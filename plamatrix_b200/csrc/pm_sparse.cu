@@ -5,8 +5,8 @@
 // synchronises with the host after every iteration.  Here:
 //   * the int64 CSR structure is validated once and kept as int32 (4 B per index on the
 //     HBM stream instead of 8 B);
-//   * SpMV uses a sub-warp per row (width chosen from the mean row length) with shuffle
-//     reductions;
+//   * SpMV takes rows of up to eight nonzeros on average 32 at a time through shared memory, a
+//     lane per row, and longer ones with 16 or 32 lanes per row and shuffle reductions;
 //   * a CG / PCG solve is one cooperative kernel where that is the faster form (pcg_row_kernel,
 //     pcg_loop_kernel): SpMV with the p.q dot, vector update with preconditioner apply and the
 //     r.z / r.r dots, direction, with grid barriers between.  Elsewhere the same three steps are
@@ -417,9 +417,9 @@ __global__ void __launch_bounds__(256) csr_spmv_kernel(int64_t rows, const int* 
     }
 }
 
-// heuristic lanes per row: a thread per row up to 8 nonzeros per row on average (its grouped
-// loads beat the row-group stream there: 49 vs 61 us on the 128^3 Laplacian), then the next
-// power of two above the mean
+// heuristic lanes per row: a lane per row up to 8 nonzeros per row on average (128^3 Laplacian FP64, cold:
+// 39 us from staged tiles, 45 read in groups where the values are not aligned, 56 as a row-group stream),
+// then 16 or 32
 int pick_tpr(int64_t rows, int64_t nnz)
 {
     const double mean = rows > 0 ? double(nnz) / double(rows) : 1.0;
@@ -527,10 +527,14 @@ struct PcgState
 //                    against 14.5)
 // Everything else runs the graph: with one CTA of at most 1,024 threads per SM the vector phases
 // of larger systems, and the block preconditioner's, have too few loads in flight (150^3 FP64: 145
-// us an iteration against 132; 24,000 rows of 474 in FP64: 55 against 49).
+// us an iteration against 132; 24,000 rows of 474 in FP64: 55 against 44).
 constexpr int kLoopThreads = kGridMaxThreads;      // most threads of a CTA (one CTA per SM)
 constexpr int kRowThreads = 512;                   // most threads of a CTA with one row per thread
-constexpr int kKeepCap = 232;                      // staged nonzeros per tile beside the kept residual (7 per row)
+// Staged nonzeros per tile beside the kept residual: 32 rows of 7.25.  What a tile takes is lost to the residual:
+// 23 entries a thread in FP64 (2.18M rows) with 232, 21 (1.99M) with 256.  Longer rows on average take a second
+// load per tile and are still faster than as kernels (30 iterations, FP64: 600,000 rows of 7.3 1.36 -> 1.14 ms,
+// of 7.9 1.42 -> 1.20; 1.5M of 7.9 2.84 -> 2.64).
+constexpr int kKeepCap = 232;
 constexpr int kTileThreads = 640;                  // of a CTA that stages tiles of the matrix
 
 template <typename T>
@@ -1852,8 +1856,9 @@ bool launch_cooperative(Kernel kernel, PcgLoop<T>& a, unsigned ctas, unsigned th
 // that read directly).  Jacobi PCG, 30 iterations, us, as kernels / rows in registers / staged tiles with the
 // kept residual: 60,000 rows of 5 and one of 128, FP64 748 / 600 / 508, FP32 701 / 443 / 452; one of 1,000,
 // 2,555 / 2,753 / 1,214 and 2,104 / 1,711 / 986.  Blocks of six, FP32, one of 1,000: one launch 2,166,
-// kernels 1,437; FP64 1,935 and 2,469.
+// kernels 1,437; FP64 1,935 and 2,469, but one of 12,000 25.2 ms and 24.0.
 constexpr int kLoneRow = 128;
+constexpr int kLoneBlockRow = 8192;
 
 template <typename T, int SHAPE>
 bool launch_pcg_loop_shape(PcgLoop<T>& a, size_t warp_smem, int lanes, int longest_row, cudaStream_t stream)
@@ -1886,7 +1891,7 @@ bool launch_pcg_loop_shape(PcgLoop<T>& a, size_t warp_smem, int lanes, int longe
             return launch_cooperative(pcg_loop_kernel<T, 1, true>, a, ctas, kTileThreads, staged + kept, kSmem, stream);
         warp_smem = 2 * sizeof(RowTile<T, kTileCap>);
     }
-    if ((SHAPE == -1 || (SHAPE == 1 && sizeof(T) == 4)) && longest_row > kLoneRow)
+    if ((SHAPE == -1 || SHAPE == 1) && longest_row > (SHAPE == 1 && sizeof(T) == 8 ? kLoneBlockRow : kLoneRow))
         return false;
     // few lanes: one row per thread (or group of lanes)
     constexpr unsigned kMost = loop_threads<T>(SHAPE);
