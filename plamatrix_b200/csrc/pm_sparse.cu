@@ -436,10 +436,14 @@ int pick_tpr(int64_t rows, int64_t nnz)
 // FP32 22.7 -> 16.5 us, FP64 50.6 -> 28.9; 12,000 of 1,000, FP32 25.0 -> 16.5, FP64 57.5 -> 28.8.  Below that
 // most of a round is empty and half the warps are gone: 24,000 rows of 400, 30 FP32 iterations 833 us one
 // after the other against 880; 240,000 rows of 32, FP64 57 us against 97; an 80^3 27-point grid 112 against 213.
+// A lone long row is a chain of its own, 6 ns a nonzero less in rounds; the rest pays 0.007 ns a nonzero of the
+// matrix: 60,000 rows of 18, FP64, one of 5,000, 45 us one after the other and 21 in rounds; 240,000 rows of
+// 18, one of 5,000, 47 and 72, one of 20,000, 168 and 72.
 inline bool long_rows(const pm_csr* A)
 {
-    return lanes_per_row(A) == 32 && A->nnz >= 14 * 32 * A->rows &&
-           A->nnz <= INT32_MAX - 8 * 32; // positions a round past the end fit in an int
+    if (lanes_per_row(A) != 32 || A->nnz > INT32_MAX - 8 * 32) // positions a round past the end fit in an int
+        return false;
+    return A->nnz >= 14 * 32 * A->rows || (A->longest_row >= 256 && A->nnz <= 512 * int64_t(A->longest_row));
 }
 
 // one lane per row from staged tiles: the values (the caller's array) on a 16-byte boundary

@@ -126,3 +126,15 @@ def test_one_long_row(checkers, dtype, n, longest):
     matrix = _symmetric(lengths, longest)
     assert np.diff(matrix[0]).max() == longest
     _check(checkers, matrix, dtype, ("pcg", "cg", "block_pcg"))
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("n", [700, 5000])
+@pytest.mark.parametrize("longest", [100, 270, 600])
+def test_one_long_row_among_longer_ones(checkers, dtype, n, longest):
+    """Rows of 21 and one of 100 to 600: the lanes of every row read one after the other, or in rounds."""
+    lengths = np.full(n, 21)
+    lengths[n // 2] = 2 * (longest - 11) + 1
+    matrix = _symmetric(lengths, longest)
+    assert np.diff(matrix[0]).max() == longest
+    _check(checkers, matrix, dtype, ("pcg", "cg"))
