@@ -142,20 +142,21 @@ __device__ __forceinline__ bool grid_barrier(GridSync& g)
 }
 
 // The mailboxes of one workspace and the number below which all its barriers lie so far, zeroed once.  Every
-// launch takes numbers of its own from the device, through grid_next_launch in a kernel queued before it: a
-// captured launch is replayed with the same arguments, and packets of the replay before must not pass for its own.
+// launch takes numbers of its own.  One that may be captured takes them on the device, through grid_next_launch
+// in a kernel queued before it: it is replayed with the same arguments, and packets of the replay before must not
+// pass for its own.  A workspace whose solves wait on the host, and so are never captured, takes next_launch().
 constexpr size_t kGridPackets = 4 * size_t(kGridMaxCtas) * kGridMaxCtas;
+constexpr unsigned long long kGridEpochs = 1ull << 34; // more than the barriers of any solve (three per iteration)
 
-__device__ __forceinline__ void grid_next_launch(unsigned long long* epoch)
-{
-    *epoch += 1ull << 34; // more than the barriers of any solve (three per iteration)
-}
+__device__ __forceinline__ void grid_next_launch(unsigned long long* epoch) { *epoch += kGridEpochs; }
 
 struct GridMail
 {
     DeviceBuffer buffer;
     Packet* packets() const { return static_cast<Packet*>(buffer.ptr); }
     unsigned long long* epoch() const { return reinterpret_cast<unsigned long long*>(packets() + kGridPackets); }
+    unsigned long long launches = 0;
+    unsigned long long next_launch() { return ++launches * kGridEpochs; }
     void open(cudaStream_t stream, const char* owner)
     {
         buffer.bind(stream, owner);

@@ -1656,7 +1656,7 @@ struct SchurLoop
     const SchurStatus* status; // factorisations to have succeeded, or null
     int64_t observations;
     Packet* mail;
-    const unsigned long long* epoch;
+    unsigned long long epoch;
     SolveState* st;
 };
 
@@ -1664,12 +1664,6 @@ __device__ __forceinline__ bool schur_status_bad(const SchurStatus* s, int64_t o
 {
     return s->eliminated_bad != kNone || s->preconditioner_bad != kNone ||
            (s->observation_bad >= 0 && s->observation_bad < observations);
-}
-
-__global__ void solve_reset_kernel(SolveState* st, unsigned long long* epoch)
-{
-    *st = SolveState{};
-    grid_next_launch(epoch);
 }
 
 // ROWS: the most rows (warps) of a CTA, which gives a thread 214, 128, 80 or 64 registers with 8, 16, 24 or 32: the
@@ -1683,7 +1677,7 @@ __global__ void __launch_bounds__(32 * ROWS, 1) schur_pcg_kernel(const SchurLoop
     if (a.status && schur_status_bad(a.status, a.observations))
         return; // nothing is solved; the host reports why
     SolveState* const st = a.st;
-    GridSync sync{a.mail, &st->timed_out, &shared, *a.epoch};
+    GridSync sync{a.mail, &st->timed_out, &shared, a.epoch};
     if (threadIdx.x == 0)
         shared.failed = 0; // read after the first barrier's __syncthreads
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -3166,7 +3160,7 @@ bool queue_one_launch_pcg(pm_schur_workspace* ws, cudaStream_t stream, const M* 
     ws->mail.open(stream, "SchurComplementSolverWorkspace");
     SchurLoop<V, M, PM> a{ws->P, ws->block_row_ptr, ws->block_col, S, minv, rhs, x, scratch, rel, abs_tol, rule,
                           max_iterations, window, x_is_zero, check, status, observations, ws->mail.packets(),
-                          ws->mail.epoch(), ws->state};
+                          ws->mail.next_launch(), ws->state};
     // One CTA while it holds all rows (its barriers are the cheapest), else at least eight rows each.  Rows
     // longer than a warp's one round of loads are spread over all SMs; shorter ones take fewer CTAs, in steps
     // of eight, because the barriers cost more than the loads (1,500 rows of 18 blocks, mixed precision: 309 us
@@ -3180,8 +3174,7 @@ bool queue_one_launch_pcg(pm_schur_workspace* ws, cudaStream_t stream, const M* 
         if (ws->B <= 32 * ws->P || rows > 24)
             rows = (rows + 7) / 8 * 8;
     }
-    solve_reset_kernel<<<1, 1, 0, stream>>>(ws->state, ws->mail.epoch());
-    PM_LAUNCH_CHECK();
+    PM_CUDA(cudaMemsetAsync(ws->state, 0, sizeof(SolveState), stream));
     const auto kernel = rows <= 8    ? schur_pcg_kernel<V, M, PM, 8>
                         : rows <= 16 ? schur_pcg_kernel<V, M, PM, 16>
                         : rows <= 24 ? schur_pcg_kernel<V, M, PM, 24>
