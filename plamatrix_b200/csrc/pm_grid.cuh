@@ -148,7 +148,8 @@ __device__ __forceinline__ bool grid_barrier(GridSync& g)
 constexpr size_t kGridPackets = 4 * size_t(kGridMaxCtas) * kGridMaxCtas;
 constexpr unsigned long long kGridEpochs = 1ull << 34; // more than the barriers of any solve (three per iteration)
 
-__device__ __forceinline__ void grid_next_launch(unsigned long long* epoch) { *epoch += kGridEpochs; }
+// an atomic without a result, which the kernel does not wait for
+__device__ __forceinline__ void grid_next_launch(unsigned long long* epoch) { atomicAdd(epoch, kGridEpochs); }
 
 struct GridMail
 {
