@@ -149,6 +149,10 @@ PM_API int pm_csr_create_f32(pm_stream_t stream, int64_t rows, int64_t cols, int
                       const int64_t* col_indices_d, const float* values_d, pm_csr** out);
 PM_API int pm_csr_create_f64(pm_stream_t stream, int64_t rows, int64_t cols, int64_t nnz, const int64_t* row_offsets_d,
                       const int64_t* col_indices_d, const double* values_d, pm_csr** out);
+/* Destroying a handle does not wait for kernels that were queued with it.  pm_csr_wait does: it synchronises
+ * the streams on which products or fixed-iteration solves were queued (which must still exist), except those
+ * that are being captured, whose graph needs the handle as long as it is replayed. */
+PM_API int pm_csr_wait(const pm_csr* matrix);
 PM_API void pm_csr_destroy(pm_csr* matrix);
 /* Point the handle at new values with the same structure (e.g. the next LM iteration). */
 PM_API int pm_csr_set_values(pm_csr* matrix, const void* values_d);

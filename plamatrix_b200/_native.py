@@ -94,6 +94,7 @@ _SIGNATURES = {
     "pm_coo_to_csr_static_f64": [vp, i64, i64, i64, vp, vp, vp, i64, vp, vp, vp, vp],
     "pm_csr_create_f32": [vp, i64, i64, i64, vp, vp, vp, vp],
     "pm_csr_create_f64": [vp, i64, i64, i64, vp, vp, vp, vp],
+    "pm_csr_wait": [vp],
     "pm_csr_destroy": [vp],
     "pm_csr_set_values": [vp, vp],
     "pm_csr_spmv_f32": [vp, vp, vp, vp],

@@ -17,10 +17,13 @@
 #include "pm_grid.cuh"
 #include "pm_piece.h"
 
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <limits>
+#include <mutex>
 #include <sstream>
+#include <vector>
 
 struct pm_csr
 {
@@ -33,6 +36,15 @@ struct pm_csr
     int longest_row = 0;     // its nonzeros
     uint64_t serial = 0;     // no other operand of the process has it, also none that is created later
     int kernel = -1;         // -1: heuristic; 0: row-group stream; 1..32: lanes per row (autotuned or set)
+    // streams on which products or fixed-iteration solves were queued (pm_csr_wait)
+    mutable std::mutex used_lock;
+    mutable std::vector<cudaStream_t> used;
+    void queued_on(cudaStream_t stream) const
+    {
+        const std::lock_guard<std::mutex> lock(used_lock);
+        if (std::find(used.begin(), used.end(), stream) == used.end())
+            used.push_back(stream);
+    }
 };
 
 namespace pm
@@ -1509,6 +1521,7 @@ void csr_spmv(const pm_csr* A, cudaStream_t stream, const T* x, T* y)
         fail(PM_INVALID_ARGUMENT, "spmv vectors must be non-null");
     if (x && x == y)
         fail(PM_INVALID_ARGUMENT, "spmv input and output data must not alias");
+    A->queued_on(stream);
     launch_spmv<T>(A, x, y, stream);
 }
 
@@ -1687,6 +1700,7 @@ void csr_spmm(const pm_csr* A, cudaStream_t stream, int64_t in_rows, int64_t in_
         PM_CUDA(cudaMemsetAsync(out, 0, size_t(out_rows * out_cols) * sizeof(T), stream));
         return;
     }
+    A->queued_on(stream);
     csr_spmm_kernel<T><<<grid_for(A->rows, 256, 1 << 20), 256, 0, stream>>>(A->rows, A->cols, in_cols, A->row_ptr,
                                                                              A->col_idx, static_cast<const T*>(A->values),
                                                                              in, out);
@@ -2082,6 +2096,7 @@ pm_fixed_state* fixed_solve(pm_solver_workspace* ws, cudaStream_t stream, const 
             PM_CUDA(cudaEventRecord(state->event, stream));
             return state;
         }
+        A->queued_on(stream);
         const PcgState* st = queue_pcg<T>(ws, A, b, x, static_cast<const T*>(nullptr), 0, mode, 0.0, 0.0, iterations,
                                           false, stream);
         fixed_finish_kernel<<<1, 1, 0, stream>>>(st, state->residuals);
@@ -2179,12 +2194,30 @@ void pm_csr_destroy(pm_csr* A)
 {
     if (A)
     {
-        // stream-ordered memory: cudaFree does not wait for the kernels that still read it
-        cudaDeviceSynchronize();
-        cudaFree(A->row_ptr);
+        cudaFree(A->row_ptr); // stream-ordered memory: it does not wait for kernels that still read it
         cudaFree(A->col_idx);
         delete A;
     }
+}
+int pm_csr_wait(const pm_csr* A)
+{
+    return pm::guarded([&] {
+        if (!A)
+            pm::fail(PM_INVALID_ARGUMENT, "CSR handle is null");
+        std::vector<cudaStream_t> streams;
+        {
+            const std::lock_guard<std::mutex> lock(A->used_lock);
+            streams.swap(A->used);
+        }
+        for (const cudaStream_t stream : streams)
+        {
+            cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+            if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess)
+                cudaGetLastError(); // the legacy stream beside a capture: it cannot be waited for either
+            else if (capture == cudaStreamCaptureStatusNone)
+                PM_CUDA(cudaStreamSynchronize(stream));
+        }
+    });
 }
 int pm_csr_set_values(pm_csr* A, const void* values)
 {

@@ -221,6 +221,7 @@ class CsrOperand:
         h = getattr(self, "_h", None)
         try:
             if h is not None and N._lib is not None:
+                N._lib.pm_csr_wait(h)  # a product may still be queued
                 N._lib.pm_csr_destroy(h)
         except (AttributeError, TypeError):  # interpreter shutdown
             pass

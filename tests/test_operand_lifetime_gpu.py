@@ -32,3 +32,35 @@ def test_operand_dropped_behind_queued_work(dtype):
         del taken
     y = S.spmv(matrix, x)
     assert bool(((y.double() - want).abs() <= (width + 1) * torch.finfo(dtype).eps * want).all())
+
+
+def test_operand_dropped_during_a_capture():
+    """Another operand with work queued on another stream is dropped while a stream is captured (relaxed mode,
+    in which memory may be released): the capture goes on and replays."""
+    n = 10_000
+    offsets, columns = torch.arange(n + 1, device="cuda"), torch.arange(n, device="cuda")
+    values, x = torch.rand(n, dtype=torch.float64, device="cuda"), torch.rand(n, dtype=torch.float64, device="cuda")
+    y, z = torch.zeros_like(x), torch.zeros_like(x)
+    kept, dropped = (S.CsrOperand(S.CSRMatrix(n, n, offsets, columns, values)) for _ in range(2))
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    dropped.spmv(x, z)
+    kept.spmv(x, y)
+    torch.cuda.synchronize()
+    dropped.spmv(x, z)
+    with torch.cuda.stream(stream):
+        graph.capture_begin(capture_error_mode="relaxed")
+        dropped.spmv(x, z)
+        kept.spmv(x, y)
+        graph.capture_end()
+        graph.reset()
+        dropped.spmv(x, z)
+        graph = torch.cuda.CUDAGraph()
+        graph.capture_begin(capture_error_mode="relaxed")
+        kept.spmv(x, y)
+        del dropped
+        kept.spmv(x, y)
+        graph.capture_end()
+        y.zero_()
+        graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, values * x) and torch.equal(z, values * x)
