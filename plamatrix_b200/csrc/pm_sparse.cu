@@ -167,7 +167,8 @@ __device__ __forceinline__ T csr_row_dot(const int* __restrict__ rp, const int* 
 // ------------------------------------------------------------------ staged row tiles
 // One lane per row with the matrix staged in shared memory.  A warp takes tiles of 32 consecutive
 // rows; the tile's nonzeros are one contiguous range of columns and values, brought in by 16-byte
-// asynchronous copies (coalesced, marked evict-first in L2 so that the vectors stay), and lane i then sums row i in storage order from shared memory.  Reading the
+// asynchronous copies (coalesced, marked evict-first in L2 so that the vectors stay), and lane i
+// then sums row i in storage order from shared memory.  Reading the
 // same rows directly costs a lane-strided access per nonzero: 180 load wavefronts per 32 rows of
 // seven FP64 nonzeros against about 100 here, and at 180 the load pipe (45 us for the 128^3
 // Laplacian) is slower than HBM.
@@ -302,7 +303,8 @@ __device__ __forceinline__ void csr_tiles(RowTile<T, CAP>* stage, int64_t rows, 
         __syncwarp();
         const int first = __shfl_sync(0xffffffffu, b, 0) & ~3;
         const int end = __shfl_sync(0xffffffffu, e, 31);
-        const T sum = tile_row<BUFFERS == 1 && sizeof(T) == 4 ? 4 : 8>(stage[buffer], ci, v, b, e, first, end, nnz, policy, lane, x_at);
+        constexpr int G = BUFFERS == 1 && sizeof(T) == 4 ? 4 : 8;
+        const T sum = tile_row<G>(stage[buffer], ci, v, b, e, first, end, nnz, policy, lane, x_at);
         if (t * 32 + lane < rows)
             done(t * 32 + lane, sum);
         __syncwarp();
@@ -623,7 +625,7 @@ __device__ __forceinline__ void jacobi_row(int64_t r, const int* __restrict__ rp
         for (int k = 0; k < G; ++k)
             if (k < left)
             {
-                most = max(most, abs(value[k]));
+                most = fmax(most, fabs(value[k]));
                 if (col[k] == r)
                 {
                     diag += static_cast<double>(value[k]);

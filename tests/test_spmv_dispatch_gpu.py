@@ -8,6 +8,7 @@ import pytest
 import torch
 
 from gpu_util import dev, host, tdtype
+from plamatrix_b200 import _native as N
 from plamatrix_b200 import sparse as S
 
 pytestmark = pytest.mark.gpu
@@ -138,3 +139,18 @@ def test_one_long_row_among_longer_ones(checkers, dtype, n, longest):
     matrix = _symmetric(lengths, longest)
     assert np.diff(matrix[0]).max() == longest
     _check(checkers, matrix, dtype, ("pcg", "cg"))
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("row", [0, 200, 399])
+def test_diagonal_near_zero(dtype, row):
+    """A diagonal entry far below its row's largest, with all values below one: the row is named.  Long and
+    short rows."""
+    n = 400
+    ro, ci, v = _symmetric(np.where(np.arange(n) % 50 == 0, 41, 5), 3)
+    v = v / np.abs(v).max() / 2.0
+    at = np.repeat(np.arange(n), np.diff(ro))
+    v[(at == row) & (ci == row)] = 4.0 * np.finfo(dtype).eps * np.abs(v[(at == row) & (ci != row)]).max()
+    x = torch.zeros(n, dtype=tdtype(dtype), device="cuda")
+    with pytest.raises(N.PlamatrixError, match=f"near zero at row {row}$"):
+        S.pcg(_operand((ro, ci, v), dtype), torch.ones_like(x), x)
