@@ -2567,14 +2567,18 @@ constexpr int kUpperShapeCount = sizeof(kUpperShapes) / sizeof(kUpperShapes[0]);
 //     blocks, FP64 243 277 246 227;
 //   four lanes a pair keep 24 instead of 16 warps per SM, which pays with FP32 rows (217.8 pairs, FP32
 //     1935 1972 1851 1859) and with fewer blocks (27 pairs, 19,900 blocks, FP64 113 113 103 113; 93 pairs,
-//     45,150 blocks, FP64 335 329 349 355; 93 pairs, 11,700 blocks, FP64 348 412 367 333);
+//     11,700 blocks, FP64 348 412 367 333; 300 pairs, 24,000 blocks, FP64 419 461 434 399; 31,375 blocks,
+//     FP64 617 651 656 656; 93 pairs, 45,150 blocks, FP64 335 329 349 355);
+//   small nearly dense systems keep two lanes a pair with FP32 rows: 600 pairs, 11,325 blocks of 150 rows, FP32
+//     322 366 411 344, FP64 466 574 454 449;
 //   below some 4,000 blocks a block's own chain is all there is: 63 pairs, 190 blocks, FP64 37 43 44 37.
 int default_shape(const pm_schur_workspace* ws, bool fp64)
 {
-    const bool split2 = fp64 && ws->U >= 32768;
-    if (ws->E < 64 * ws->U && ws->U >= 4096)
-        return split2 ? 1 : 3;
-    return split2 ? 0 : 4;
+    const bool many_pairs = ws->E >= 64 * ws->U, many_blocks = ws->U >= 28672;
+    if (!many_pairs && ws->U >= 4096)
+        return fp64 && many_blocks ? 1 : 3;
+    const bool small_dense = ws->U >= 4096 && !many_blocks && 4 * ws->U > ws->P * ws->P;
+    return (fp64 ? many_blocks : small_dense) ? 0 : 4;
 }
 
 template <typename TO, typename TP, typename VT, typename AT, int STREAMS, int SPLIT>
